@@ -69,6 +69,10 @@ Consts make_consts(const nsf_config& c, const HostSetup& s) {
   K.dy = dy;
   K.dz = dz;
   K.dxdydz = dx * dy * dz;
+  {
+    const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
+    K.invD2 = 1 / dx2 + 1 / dy2 + 1 / dz2;
+  }
   K.ax = -1. / (2 * dx);
   K.ay = -1. / (2 * dy);
   K.az = -1. / (2 * dz);

@@ -26,6 +26,7 @@ constexpr int MAX_HIST = 1 << 20;  // per-step history rows kept on the device (
 struct Consts {
   double gamma, gm1, pr, re, sc1, pf, h0, vmod, convLim, viscLim, m0, tEnd;
   double dx, dy, dz, dxdydz;
+  double invD2;  // 1/dx^2 + 1/dy^2 + 1/dz^2
   // continuity / inviscid: -1/(2d)
   double ax, ay, az;
   // x-momentum: 2/(3dx^2), 1/(2dy^2), 1/(2dz^2), -1/(6dydx), 1/(4dxdy), -1/(6dzdx), 1/(4dxdz)

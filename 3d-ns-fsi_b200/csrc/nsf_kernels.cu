@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cuda_runtime.h>
 
+#include "nsf_bc_items.cuh"
 #include "nsf_device.cuh"
 #include "nsf_internal.h"
 #include "nsf_physics.cuh"
@@ -25,94 +26,11 @@
 namespace nsf {
 
 // ----------------------------------------------------------------------------------------------
-// Prologue: Simulation::checkStoppingCriterion (end_time), Mesh::checkFilterCondition (Mesh.cpp:85-103),
-// the buffer swaps of Mesh.cpp:133-151 expressed as role changes, and per-stage buffer roles.
-// Member m = blockIdx.x of the grid array (a single grid: one block).
+// Start of a step (prologue_warp). Member m = blockIdx.x of the grid array (a single grid: one block).
 __global__ void k_prologue(Grid* grids) {
-  if (threadIdx.x != 0) return;
-  Grid* g = grids + blockIdx.x;
-  StepCtl* c = g->ctl;
-  for (int f = 0; f < 5; ++f) g->normPart[f] = 0.0;  // slot 0: the ensemble stage kernel adds into it
-  const Consts& C = g->C;
-  c->active = C.endTime ? (c->t < C.tEnd) : 1;
-  if (!c->active) return;
-  int counter = 0;
-  for (int q = 0; q < C.nChange; ++q)
-    if (c->t > C.changeT[q]) ++counter;
-  int filt = 0;
-  if (counter < C.nFilterIv) {
-    unsigned iv = C.filterIv[counter];
-    if (iv > 0 && (c->level + 1) % iv == 0) filt = 1;
-  }
-  c->filterNow = filt;
-  int cons[5], old[5], scr[5];
-  for (int f = 0; f < 5; ++f) {
-    cons[f] = c->perm[f][0];
-    old[f] = c->perm[f][1];
-    scr[f] = c->perm[f][2];
-  }
-  if (filt) {  // the filter writes rho into the old buffer, then the two rho buffers trade places
-    c->gfSrc = g->bufs[cons[0]][0];
-    c->gfDst = g->bufs[old[0]][0];
-    int t = cons[0];
-    cons[0] = old[0];
-    old[0] = t;
-  }
-  for (int f = 0; f < 5; ++f) {  // swapConservedVariables
-    int t = cons[f];
-    cons[f] = old[f];
-    old[f] = t;
-  }
-  int A[5], B[5];
-  for (int f = 0; f < 5; ++f) {
-    A[f] = cons[f];
-    B[f] = scr[f];
-  }
-  if (filt) {  // stage 1 cannot write the unfiltered density it reads: it writes the scratch buffer
-    A[0] = scr[0];
-    B[0] = cons[0];
-  }
-  for (int f = 0; f < 5; ++f) {
-    c->u0Phys[f] = old[f];
-    c->iPhys[0][f] = old[f];
-    c->iPhys[1][f] = A[f];
-    c->iPhys[2][f] = B[f];
-    c->iPhys[3][f] = A[f];
-  }
-  c->rPhys[0] = filt ? cons[0] : old[0];
-  c->rPhys[1] = A[0];
-  c->rPhys[2] = B[0];
-  c->rPhys[3] = A[0];
-  for (int f = 0; f < 5; ++f) {
-    c->U0[f] = g->bufs[old[f]][f];
-    c->I[0][f] = g->bufs[old[f]][f];
-    c->O[0][f] = g->bufs[A[f]][f];
-    c->I[1][f] = g->bufs[A[f]][f];
-    c->O[1][f] = g->bufs[B[f]][f];
-    c->I[2][f] = g->bufs[B[f]][f];
-    c->O[2][f] = g->bufs[A[f]][f];
-    c->I[3][f] = g->bufs[A[f]][f];
-    c->O[3][f] = g->bufs[B[f]][f];
-  }
-  c->R[0] = filt ? g->bufs[cons[0]][0] : g->bufs[old[0]][0];
-  c->R[1] = g->bufs[A[0]][0];
-  c->R[2] = g->bufs[B[0]][0];
-  c->R[3] = g->bufs[A[0]][0];
-  c->copyMask[0] = filt ? 1 : 0;
-  c->copyMask[1] = c->copyMask[2] = c->copyMask[3] = 31;
-  const double dt = c->dt;
-  c->dtUsed = dt;
-  c->stageT[0] = c->t + dt / 2;
-  c->stageT[1] = c->t + dt / 2;
-  c->stageT[2] = c->t + dt;
-  c->stageT[3] = c->t + dt;
-  for (int f = 0; f < 5; ++f) {  // roles after the step: final state = B, scratch = A
-    c->perm[f][0] = B[f];
-    c->perm[f][1] = old[f];
-    c->perm[f][2] = A[f];
-  }
-  for (int q = 0; q < 4; ++q) c->mx[q] = 0ull;
-  if (g->ctlHist && c->level < (unsigned long long)g->nCtlHist) g->ctlHist[c->level] = *c;
+  const Grid& G = grids[blockIdx.x];
+  if (threadIdx.x < 5) G.normPart[threadIdx.x] = 0.0;  // slot 0: the ensemble stage kernel adds into it
+  prologue_warp(G, G.ctl, threadIdx.x, true);
 }
 
 // Mesh::applyFilter_ifAppropriate body (Mesh.cpp:110-134): interior nodes get the 7-point filter,
@@ -122,36 +40,10 @@ __global__ void k_density_filter(const Grid* __restrict__ grids) {
   const Grid* g = grids + blockIdx.y;
   const StepCtl* c = g->ctl;
   if (!c->active || !c->filterNow) return;
-  const double* __restrict__ src = c->gfSrc;
-  double* __restrict__ dst = c->gfDst;
-  const long long sI = g->sI, sJ = g->sJ;
-  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < g->N; n += (long long)gridDim.x * blockDim.x) {
-    const uint8_t raw = g->type[n], t = raw & TYPE_MASK;
-    if (t == FLUID_INTERIOR)
-      dst[n] = (6 * src[n] + src[n + sI] + src[n - sI] + src[n + sJ] + src[n - sJ] + src[n + 1] + src[n - 1]) / 12;
-    else if (t != SOLID_INACTIVE || (raw & EDGE_PLANE_BIT))
-      dst[n] = src[n];
-  }
+  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < g->N; n += (long long)gridDim.x * blockDim.x)
+    density_filter_node(*g, c, n);
 }
 
-// ----------------------------------------------------------------------------------------------
-// Solid-node values the reference's stage buffer still holds from earlier writes (see nsf_device.cuh).
-// One solid node q of a grid; the device functions here are shared by the separate kernels and the fused
-// boundary kernel (k_bc), which reads fields written earlier in the same launch: those reads bypass L1.
-__device__ __forceinline__ void solid_copy_item(const Grid& G, const StepCtl* c, int s, int mask, int q) {
-  const long long n = G.snode[q];
-  if (mask & 1) c->O[s][0][n] = __ldcg(c->R[s] + n);
-  for (int f = 1; f < 5; ++f)
-    if (mask & (1 << f)) c->O[s][f][n] = __ldcg(c->I[s][f] + n);
-}
-
-// Field f at node m as the stage's boundary work reads it after the solid-node copy. For a solid node off
-// the mesh faces (solid = true; nothing but the copy writes it in a stage) the value comes from the copy's
-// source, so the reader does not wait for the copy; the values are the same either way.
-__device__ __forceinline__ double ld_res(const StepCtl* c, int s, int f, long long m, bool solid) {
-  if (solid && (c->copyMask[s] & (1 << f))) return __ldcg((f == 0 ? c->R[s] : c->I[s][f]) + m);
-  return __ldcg(c->O[s][f] + m);
-}
 
 __global__ void k_solid_copy(const Grid* __restrict__ grids, int s) {
   const Grid* g = grids + blockIdx.y;
@@ -163,140 +55,6 @@ __global__ void k_solid_copy(const Grid* __restrict__ grids, int s) {
     solid_copy_item(*g, c, s, mask, q);
 }
 
-// ----------------------------------------------------------------------------------------------
-// Mesh-edge boundary conditions of one axis (both faces; the faces of one axis never read each other's
-// nodes). Launched for x, then y, then z: the reference's application order outlet/inlet (x), y-max,
-// y-min, z-max, z-min (Mesh.cpp:155-167 after the reversal at Mesh.cpp:70). Each block comes from the
-// launch plan's list (member, face, first in-plane coordinates, mask of the nodes it works on).
-// periodic_source: the node a periodic face node finally copies -- the opposite interior-plane node, and if
-// that node lies on another periodic face (which copied it earlier in the reference's order), that face's
-// source, and so on (at most two more hops). The copies are exact, so reading the final source gives the
-// value the reference copies; it lets chains of copies run together (nsf_bc_plan.cpp).
-// edge_node: one node (thread tx, ty of an edge block) of a mesh-edge boundary condition; adds the stage-4
-// dt terms and the NaN check of edge and ghost-typed nodes.
-__device__ __forceinline__ void periodic_source(const Grid& G, int axis, int side, int ijk[3]) {
-  const int nAx[3] = {G.NI, G.NJ, G.NK};
-  ijk[axis] = side == 0 ? nAx[axis] - 2 : 1;
-  for (int hop = 0; hop < 2; ++hop) {
-    int found = -1;
-    for (int e = 0; e < G.nEdge && found < 0; ++e) {
-      const int* b = G.eBox[e];
-      if (G.eBc[e] == NSF_BC_PERIODIC && ijk[0] >= b[0] && ijk[0] <= b[1] && ijk[1] >= b[2] && ijk[1] <= b[3] &&
-          ijk[2] >= b[4] && ijk[2] <= b[5])
-        found = e;
-    }
-    if (found < 0) return;
-    const int a = G.eAxis[found];
-    ijk[a] = G.eSide[found] == 0 ? nAx[a] - 2 : 1;
-  }
-}
-
-__device__ __forceinline__ void edge_node(const Grid& G, const StepCtl* c, const EdgeBlock& eb, int tx, int ty, int s,
-                                          int axis, DtAcc& dta, int& bad) {
-  const Consts& C = G.C;
-  const int e = eb.e;
-  {
-    const int* b = G.eBox[e];
-    // in-plane coordinates: (a, bb) = the two axes other than `axis`, in (i, j, k) order
-    const int ax1 = axis == 0 ? 1 : 0, ax2 = axis == 2 ? 1 : 2;
-    const int a = eb.a0 + ty;
-    const int bb = eb.b0 + tx;
-    if (a <= b[2 * ax1 + 1] && bb <= b[2 * ax2 + 1] && ((eb.mask >> (ty * 32 + tx)) & 1)) {
-      int ijk[3];
-      ijk[axis] = b[2 * axis];
-      ijk[ax1] = a;
-      ijk[ax2] = bb;
-      const long long st = axis == 0 ? G.sI : axis == 1 ? G.sJ : 1;
-      const long long n = ijk[0] * G.sI + ijk[1] * G.sJ + ijk[2];
-      const int side = G.eSide[e], bc = G.eBc[e];
-      double* const* O = c->O[s];
-      const bool solidSrc = (eb.solidSrc >> (ty * 32 + tx)) & 1;
-      auto ld = [&](int f, long long m) { return ld_res(c, s, f, m, solidSrc); };
-      const long long a1 = side == 0 ? n + st : n - st, a2 = side == 0 ? n + 2 * st : n - 2 * st;  // Boundary.cpp:74-108
-      double cv[5];
-      double u = 0, v = 0, w = 0, p = 0, T = 0;
-      bool primKnown = false;
-      if (bc == NSF_BC_INLET) {  // Boundary.cpp:250-296 with filterInletDensity :142-245
-        // extrapolated density of this node and of its in-plane neighbours inside the owned box
-        const long long s1 = ax1 == 0 ? G.sI : G.sJ, s2 = ax2 == 1 ? G.sJ : 1;
-        auto ext = [&](long long m) { return 2 * ld(0, side == 0 ? m + st : m - st) - ld(0, side == 0 ? m + 2 * st : m - 2 * st); };
-        double f = 0;
-        unsigned nn = 0;
-        if (a < b[2 * ax1 + 1]) { f += ext(n + s1); ++nn; }
-        if (a > b[2 * ax1]) { f += ext(n - s1); ++nn; }
-        if (bb < b[2 * ax2 + 1]) { f += ext(n + s2); ++nn; }
-        if (bb > b[2 * ax2]) { f += ext(n - s2); ++nn; }
-        f += nn * ext(n);
-        f /= 2 * nn;
-        const double rho = f;
-        double vel = fmin(1., c->stageT[s] / 10.) * C.m0;
-        if (G.inflow && axis == 0) vel *= G.inflow[a * G.NKp + bb];  // profile factor (1 in a plain run)
-        if (side == 1) vel *= -1;
-        u = axis == 0 ? vel : 0;
-        v = axis == 1 ? vel : 0;
-        w = axis == 2 ? vel : 0;
-        T = 0;
-        p = (T * (1 + rho) + rho) / C.gamma;
-        cons_of(C, u, v, w, p, T, cv);
-        primKnown = true;
-      } else if (bc == NSF_BC_OUTLET) {  // Boundary.cpp:304-336
-        const double rho = 2 * ld(0, a1) - ld(0, a2);
-        const double ru = 2 * ld(1, a1) - ld(1, a2);
-        const double rv = 2 * ld(2, a1) - ld(2, a2);
-        const double rw = 2 * ld(3, a1) - ld(3, a2);
-        p = 0;
-        u = ru / (1 + rho);
-        v = rv / (1 + rho);
-        w = rw / (1 + rho);
-        T = (C.gamma * p - rho) / (1 + rho);
-        cv[0] = rho;
-        cv[1] = ru;
-        cv[2] = rv;
-        cv[3] = rw;
-        cv[4] = p / C.gm1 + (1 + rho) / 2 * (u * u + v * v + w * w);
-        primKnown = true;
-      } else if (bc == BC_SLAB_COPY) {  // an x-slab's periodic x face: already copied by the plane exchange
-        for (int f = 0; f < 5; ++f) cv[f] = ld(f, n);
-      } else if (bc == NSF_BC_PERIODIC) {  // Boundary.cpp:344-367, opposite index :111-133
-        int src[3] = {ijk[0], ijk[1], ijk[2]};
-        periodic_source(G, axis, side, src);
-        const long long m = src[0] * G.sI + src[1] * G.sJ + src[2];
-        for (int f = 0; f < 5; ++f) cv[f] = ld(f, m);
-      } else {  // symmetry, Boundary.cpp:377-417: mirror the primitives of the second interior node
-        const Prim q = prims_of(C, ld(0, a2), ld(1, a2), ld(2, a2), ld(3, a2), ld(4, a2));
-        u = q.u;
-        v = q.v;
-        w = q.w;
-        if (axis == 0) u = -q.u;
-        if (axis == 1) v = -q.v;
-        if (axis == 2) w = -q.w;
-        p = q.p;
-        T = q.T;
-        cons_of(C, u, v, w, p, T, cv);
-        primKnown = true;
-      }
-      for (int f = 0; f < 5; ++f) O[f][n] = cv[f];
-      if (s == 3) {
-        const uint8_t t = G.type[n] & TYPE_MASK;
-        if (t == FLUID_EDGE || t == FLUID_GHOST) {
-          double mu;
-          if (primKnown) {
-            mu = mu_of_T(C, T);
-          } else {
-            const Prim q = prims_of(C, cv[0], cv[1], cv[2], cv[3], cv[4]);
-            u = q.u;
-            v = q.v;
-            w = q.w;
-            p = q.p;
-            mu = q.mu;
-          }
-          dta.add(C, cv[0], u, v, w, p, mu);
-          for (int f = 0; f < 5; ++f) bad |= !isfinite(cv[f]);
-        }
-      }
-    }
-  }
-}
 
 __global__ void k_edge_bc(const Grid* __restrict__ grids, const EdgeBlock* __restrict__ blocks, int s, int axis) {
   __shared__ double red[4 * 32];
@@ -313,43 +71,6 @@ __global__ void k_edge_bc(const Grid* __restrict__ grids, const EdgeBlock* __res
   }
 }
 
-// ----------------------------------------------------------------------------------------------
-// Near-body filter (ImmersedBoundary::filterClosestFluidNodes, Boundary.cpp:618-652). Jacobi: every
-// filtered value is computed from unfiltered neighbours; results go to fnew and are written back by
-// the ghost pass. The values before the filter go to fpre: the reference does not recompute the primitive
-// variables of these nodes after filtering, so the next stage builds their primitives from fpre.
-// filter_item: filter node f of a grid (stage-4 dt terms, change norms of rho and rho_E, NaN check).
-__device__ __forceinline__ void filter_item(const Grid& G, const StepCtl* c, int s, int f, DtAcc& dta, double nsum[5],
-                                            int& bad) {
-  double* const* O = c->O[s];
-  const long long n = G.fnode[f];
-  const unsigned sb = G.fsolid ? G.fsolid[f] : 0u;
-  auto r = [&](long long m, int q) { return ld_res(c, s, 0, m, (sb >> q) & 1); };
-  auto e = [&](long long m, int q) { return ld_res(c, s, 4, m, (sb >> q) & 1); };
-  const double r0 = r(n, 0), e0 = e(n, 0);
-  const double rf =
-      (6 * r0 + r(n + G.sI, 1) + r(n - G.sI, 2) + r(n + G.sJ, 3) + r(n - G.sJ, 4) + r(n + 1, 5) + r(n - 1, 6)) / 12;
-  const double ef =
-      (6 * e0 + e(n + G.sI, 1) + e(n - G.sI, 2) + e(n + G.sJ, 3) + e(n - G.sJ, 4) + e(n + 1, 5) + e(n - 1, 6)) / 12;
-  G.fpre[2 * f] = r0;
-  G.fpre[2 * f + 1] = e0;
-  G.fnew[2 * f] = rf;
-  G.fnew[2 * f + 1] = ef;
-  // stage 4: the node's dt and change-norm terms, once, from its last slot (a node two bodies filter has
-  // two): the final filtered values, and primitives from the values before the node's first filter
-  const int meta = G.fmeta ? G.fmeta[f] : (f | FMETA_LAST);
-  if (s == 3 && (meta & FMETA_LAST)) {
-    const int first = meta & ~FMETA_LAST;
-    const double p0 = first == f ? r0 : __ldcg(G.fpre + 2 * first);
-    const double p4 = first == f ? e0 : __ldcg(G.fpre + 2 * first + 1);
-    const Prim q = prims_of(G.C, p0, __ldcg(O[1] + n), __ldcg(O[2] + n), __ldcg(O[3] + n), p4);
-    dta.add(G.C, rf, q.u, q.v, q.w, q.p, q.mu);
-    const double d0 = c->U0[0][n] - rf, d4 = c->U0[4][n] - ef;
-    nsum[0] += d0 * d0;
-    nsum[4] += d4 * d4;
-    bad |= !isfinite(rf) || !isfinite(ef);
-  }
-}
 
 __global__ void k_body_filter(const Grid* __restrict__ grids, int s) {
   __shared__ double red[5 * 32];
@@ -370,76 +91,6 @@ __global__ void k_body_filter(const Grid* __restrict__ grids, int s) {
   }
 }
 
-// Ghost nodes (Boundary.cpp:432-456): image-point value = cached weights x the 8 surrounding values
-// (Neumann weights for rho and rho_E, Dirichlet weights for the momenta, zero weight on ghost corners);
-// ghost value = image value with momentum negated (getGhostNodeBCVariables, :777-785). The ghost lists
-// are stored sorted by image-point cell, so the lanes of a warp gather overlapping corner sets; every
-// corner's five values are loaded before any is used (40 independent loads in flight per ghost) and summed
-// in corner order, skipping corners whose two weights are both zero, as the reference's sums do.
-// ghost_pass_item: item q of the ghost pass: q < nGhost a ghost, then the filter write-backs (ghosts read
-// the filtered values through fnew), then on stage 4 the solid inactive nodes' dt terms (the reference
-// never updates their primitive values).
-__device__ __forceinline__ void ghost_pass_item(const Grid& G, const StepCtl* c, int s, int q, DtAcc& dta, int& bad) {
-  double* const* O = c->O[s];
-  const Consts& C = G.C;
-  if (q < G.nGhost) {
-    const long long* cell = G.gcell + 8 * (long long)q;
-    const double* w = G.gw + 16 * (long long)q;
-    double v[8][5], wn[8], wd[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const long long cn = cell[m];
-      wn[m] = w[m];
-      wd[m] = w[8 + m];
-#pragma unroll
-      for (int f = 0; f < 5; ++f) v[m][f] = __ldcg(O[f] + cn);
-      const int fi = G.gsrc[8 * (long long)q + m];  // a filter corner: the filtered values it sees
-      if (fi >= 0) {
-        v[m][0] = __ldcg(G.fnew + 2 * fi);
-        v[m][4] = __ldcg(G.fnew + 2 * fi + 1);
-      }
-    }
-    double ip[5] = {0, 0, 0, 0, 0};
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      if (wn[m] == 0.0 && wd[m] == 0.0) continue;
-      ip[0] += wn[m] * v[m][0];
-      ip[4] += wn[m] * v[m][4];
-      ip[1] += wd[m] * v[m][1];
-      ip[2] += wd[m] * v[m][2];
-      ip[3] += wd[m] * v[m][3];
-    }
-    const double gc[5] = {ip[0], -ip[1], -ip[2], -ip[3], ip[4]};
-    const long long n = G.gnode[q];
-    for (int f = 0; f < 5; ++f) O[f][n] = gc[f];
-    if (s == 3 && G.glast[q]) {  // a node in two bodies' ghost lists: the dt terms of its final values
-      const Prim p = prims_of(C, gc[0], gc[1], gc[2], gc[3], gc[4]);
-      dta.add(C, gc[0], p.u, p.v, p.w, p.p, p.mu);
-      for (int f = 0; f < 5; ++f) bad |= !isfinite(gc[f]);
-    }
-  } else if (q < G.nGhost + G.nFilter) {
-    const int f = q - G.nGhost;
-    const long long n = G.fnode[f];
-    O[0][n] = __ldcg(G.fnew + 2 * f);
-    O[4][n] = __ldcg(G.fnew + 2 * f + 1);
-  } else {
-    const int z = q - G.nGhost - G.nFilter;
-    const long long n = G.inode[z];
-    const double* pr = G.iprim + 5 * (long long)z;
-    const double r0 = ld_res(c, s, 0, n, true);  // inactive nodes lie off the mesh faces
-    if (isnan(pr[0])) {  // periodic copy of a node whose primitives follow its conserved values
-      const Prim p = prims_of(C, r0, ld_res(c, s, 1, n, true), ld_res(c, s, 2, n, true), ld_res(c, s, 3, n, true),
-                              ld_res(c, s, 4, n, true));
-      dta.add(C, r0, p.u, p.v, p.w, p.p, p.mu);
-    } else {
-      dta.add(C, r0, pr[0], pr[1], pr[2], pr[3], pr[4]);
-    }
-  }
-}
-
-__device__ __forceinline__ int ghost_pass_count(const Grid& G, int s) {
-  return G.nGhost + G.nFilter + (s == 3 ? G.nInactive : 0);
-}
 
 __global__ void k_ghost(const Grid* __restrict__ grids, int s) {
   __shared__ double red[4 * 32];
@@ -458,40 +109,6 @@ __global__ void k_ghost(const Grid* __restrict__ grids, int s) {
   }
 }
 
-// ----------------------------------------------------------------------------------------------
-// End of step: change norms (Mesh::getNormOfChange, Mesh.cpp:171-178), next dt
-// (Solver::updateTimeStepSize, Solver.cpp:80-126), t += dt, ++timeLevel, history row. Called by every
-// thread of one block (block reductions); red: 5 x 32 doubles of shared memory.
-__device__ void finalize_grid(Grid* g, double* red) {
-  __shared__ double tot[5];
-  const int nSlots = g->nNormSlots;
-  StepCtl* c = g->ctl;
-  const Consts& C = g->C;
-  double s[5] = {0, 0, 0, 0, 0};
-  for (int q = threadIdx.x; q < nSlots; q += blockDim.x)
-    for (int f = 0; f < 5; ++f) s[f] += __ldcg(g->normPart + 5 * q + f);
-  flush_norms(tot, s, red);
-  if (threadIdx.x != 0) return;
-  double mx[4];
-  for (int q = 0; q < 4; ++q) mx[q] = __longlong_as_double(static_cast<long long>(atomicAdd(&c->mx[q], 0ull)));
-  const double conv = C.convLim / (mx[0] / C.dx + mx[1] / C.dy + mx[2] / C.dz);
-  const double dx2 = C.dx * C.dx, dy2 = C.dy * C.dy, dz2 = C.dz * C.dz;
-  const double visc = C.viscLim / (mx[3] * (1 / dx2 + 1 / dy2 + 1 / dz2));
-  const double tNew = c->t + c->dtUsed;
-  double dt = (visc < conv) ? visc : conv;
-  if (C.endTime && tNew + dt > C.tEnd) dt = C.tEnd - tNew;
-  if (g->dtFrozen && c->level + 1 < (unsigned long long)g->nDtFrozen) dt = g->dtFrozen[c->level + 1];
-  double* h = g->hist + 7 * (c->level % MAX_HIST);
-  h[0] = tNew;
-  h[1] = c->dtUsed;
-  for (int f = 0; f < 5; ++f) {
-    const bool kept = (f == 0 && C.convHistory != 0) || C.convHistory == 2;
-    h[2 + f] = kept ? sqrt(C.dxdydz * tot[f]) : -1.0;
-  }
-  c->t = tNew;
-  c->dt = dt;
-  c->level += 1;
-}
 
 __global__ void k_finalize(Grid* grids) {
   __shared__ double red[5 * 32];
@@ -677,7 +294,12 @@ __global__ void k_snapshot_inactive(const Grid* __restrict__ gp, SnapSlots sl, S
 // one another, and each member runs only its own levels) and those reads go through L2 (__ldcg in the item
 // functions). The member's Grid and control block are copied to shared memory first (every item reads
 // them). Stage 4 then flushes the dt maxima, change norms and NaN flag, and the member's last block to
-// finish runs the end-of-step finalize. Every block of a member passes every barrier of that member (an
+// finish runs the end-of-step finalize. Items wait for memory, not for arithmetic, so the trips to L2 in a row are
+// what counts: an item's list entry, node and flags are resolved before the level's barrier (bc_level_item), its
+// loads all go out before the first use or store, and consecutive warps of the item range lie on different
+// blocks. Measured (us per step): sphere 48^3 148 -> 130, sphere 96^3 408 -> 384, 16 spheres 256x128x128
+// 1015 -> 985, the 64-member ensemble 4109 -> 4069 (three resident blocks instead of four: 125, 378, 982, 4096).
+// Every block of a member passes every barrier of that member (an
 // inactive member's blocks do no work), so the launch is cooperative (all blocks resident).
 
 // Resident blocks of the fused boundary kernel per SM (its registers are capped to fit): the kernel is
@@ -720,39 +342,27 @@ __global__ void __launch_bounds__(256, kBcBlocksPerSM) k_bc(Grid* grids, const _
   const Grid& G = *reinterpret_cast<const Grid*>(gsm);
   const StepCtl& cs = *reinterpret_cast<const StepCtl*>(csm);  // read-only copy for the item functions
   const bool active = cs.active != 0;
-  const int gtid = bx * blockDim.x + tid, nthr = nbx * blockDim.x;
+  // warps are numbered across the member's blocks, so that a short list of items spreads over many SMs
+  const int gtid = ((tid >> 5) * nbx + bx) * 32 + (tid & 31), nthr = nbx * int(blockDim.x);
   DtAcc dta;
   double nsum[5] = {0, 0, 0, 0, 0};
   int bad = 0;
-  const int ghostCount = ghost_pass_count(G, s);
-  // A level's items of every kind form one index range -- solid copies (level 0), edge-block threads (64
-  // per block), filter items, ghost-pass items -- and each thread takes every nthr-th index, so items of
-  // different kinds run side by side rather than one list after another.
   const int levels = P.memberLevels[g];
+  int total = 0;
+  BcItem item{BC_NONE, 0, 0, 0};  // this thread's next item
+  auto resolve = [&](int L) {
+    total = bc_level_items(G, P, g, L);
+    if (gtid < total) item = bc_level_item(G, P, g, L, gtid);
+  };
+  if (levels > 0) resolve(0);
   for (int L = 0; L < levels; ++L) {
     if (L > 0) grid_barrier(P.sync + 1 + M + g, unsigned(nbx), &c->timeout);
-    if (!active) continue;
-    const int mask = cs.copyMask[s];
-    const int nS = (L == 0 && mask) ? G.nSolid : 0;
-    const int* es = P.edgeStart + L * (M + 1) + g;
-    const int* fs = P.itemStart + (L * 2) * (M + 1) + g;
-    const int* hs = fs + (M + 1);
-    const int e0 = es[0], nE = 64 * (es[1] - e0), f0 = fs[0], nF = fs[1] - f0, h0 = hs[0], nH = hs[1] - h0;
-    const int total = nS + nE + nF + nH;
-    for (int v = gtid; v < total; v += nthr) {
-      if (v < nS) {
-        solid_copy_item(G, &cs, s, mask, v);
-      } else if (v < nS + nE) {
-        const int t = v - nS, lane = t & 63;
-        const EdgeBlock eb = P.edges[e0 + (t >> 6)];
-        edge_node(G, &cs, eb, lane & 31, lane >> 5, s, G.eAxis[eb.e], dta, bad);
-      } else if (v < nS + nE + nF) {
-        filter_item(G, &cs, s, P.items[f0 + v - nS - nE], dta, nsum, bad);
-      } else {
-        const int item = P.items[h0 + v - nS - nE - nF];
-        if (item < ghostCount) ghost_pass_item(G, &cs, s, item, dta, bad);
+    if (active)
+      for (int v = gtid; v < total;) {
+        bc_run_item<LAST>(G, cs, s, item, dta, nsum, bad);
+        if ((v += nthr) < total) item = bc_level_item(G, P, g, L, v);
       }
-    }
+    if (L + 1 < levels) resolve(L + 1);
   }
   if (s == 3) {
     flush_dt(c, dta, red);

@@ -109,6 +109,31 @@ struct DtAcc {
   }
 };
 
+// dt-limit terms of a node (getInviscidTimeStepLimit / getViscousTimeStepLimit, Solver.cpp:91-126) with one
+// reciprocal of 1 + rho for all the divisions by it, reciprocals and square roots by Newton-Raphson (recip_nr,
+// sqrt_nr). The terms only enter maxima, so their last-bit rounding moves dt by at most an ulp or two.
+// dt_terms_at: velocities, pressure and temperature known, r1 = 1 / (1 + rho).
+__device__ __forceinline__ void dt_terms_at(const Consts& C, double r1, double u, double v, double w, double p, double T,
+                                            DtAcc& a) {
+  const double x = 1.0 + T;
+  const double c = sqrt_nr((1.0 + C.gamma * p) * r1);
+  a.sx = fmax(a.sx, c + fabs(u));
+  a.sy = fmax(a.sy, c + fabs(v));
+  a.sz = fmax(a.sz, c + fabs(w));
+  a.nu = fmax(a.nu, x * sqrt_nr(x) * C.sc1 * r1 * recip_nr(C.re * (T + C.sc1)) * C.vmod);
+}
+__device__ __forceinline__ void dt_terms(const Consts& C, const double (&u)[5], DtAcc& a) {
+  const double r1 = recip_nr(u[0] + 1.0);
+  const double vx = u[1] * r1, vy = u[2] * r1, vz = u[3] * r1;
+  const double p = C.gm1 * (u[4] - (u[0] + 1.0) * 0.5 * (vx * vx + vy * vy + vz * vz));
+  const double T = (C.gamma * p - u[0]) * r1;
+  dt_terms_at(C, r1, vx, vy, vz, p, T, a);
+}
+__device__ __forceinline__ void dt_terms_known(const Consts& C, double rho, double u, double v, double w, double p,
+                                               double T, DtAcc& a) {
+  dt_terms_at(C, recip_nr(rho + 1.0), u, v, w, p, T, a);
+}
+
 __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
@@ -186,11 +211,9 @@ __device__ inline void grid_barrier(unsigned long long* S, unsigned nb, int* tim
         atomicExch(timeout, 1);
         break;
       }
-      __nanosleep(32);
     }
-    __threadfence();  // the block's later loads see what the other blocks wrote before they arrived
   }
-  __syncthreads();
+  __syncthreads();  // with the acquire: the block's later loads see what the other blocks wrote before they arrived
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -91,8 +91,7 @@ __global__ void k_slab_finalize(Grid* grids, int n, const double* __restrict__ i
     if (!c->active) continue;
     const Consts& C = gp->C;
     const double conv = C.convLim / (in[0] / C.dx + in[1] / C.dy + in[2] / C.dz);
-    const double dx2 = C.dx * C.dx, dy2 = C.dy * C.dy, dz2 = C.dz * C.dz;
-    const double visc = C.viscLim / (in[3] * (1 / dx2 + 1 / dy2 + 1 / dz2));
+    const double visc = C.viscLim / (in[3] * C.invD2);
     const double tNew = c->t + c->dtUsed;
     double dt = (visc < conv) ? visc : conv;
     if (C.endTime && tNew + dt > C.tEnd) dt = C.tEnd - tNew;

@@ -155,23 +155,6 @@ __device__ __forceinline__ void reg_alloc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// dt-limit terms of a node of the new state (getInviscidTimeStepLimit / getViscousTimeStepLimit,
-// Solver.cpp:91-126) with one reciprocal of 1 + rho for all the divisions by it, reciprocals and square
-// roots by Newton-Raphson (recip_nr, sqrt_nr). The terms only enter maxima, so their last-bit rounding
-// moves dt by at most an ulp or two.
-__device__ __forceinline__ void dt_terms(const Consts& C, const double (&u)[5], DtAcc& a) {
-  const double r1 = recip_nr(u[0] + 1.0);
-  const double vx = u[1] * r1, vy = u[2] * r1, vz = u[3] * r1;
-  const double p = C.gm1 * (u[4] - (u[0] + 1.0) * 0.5 * (vx * vx + vy * vy + vz * vz));
-  const double T = (C.gamma * p - u[0]) * r1;
-  const double x = 1.0 + T;
-  const double c = sqrt_nr((1.0 + C.gamma * p) * r1);
-  a.sx = fmax(a.sx, c + fabs(vx));
-  a.sy = fmax(a.sy, c + fabs(vy));
-  a.sz = fmax(a.sz, c + fabs(vz));
-  a.nu = fmax(a.nu, x * sqrt_nr(x) * C.sc1 * r1 * recip_nr(C.re * (T + C.sc1)) * C.vmod);
-}
-
 }  // namespace
 
 // ENS = false: one grid, passed by value (its stencil coefficients are then constant-bank operands).
