@@ -620,6 +620,42 @@ nsf_status build_device(nsf_solver* s) {
       if ((st = upload(s, &L.bcSync, zero)) != NSF_OK) return st;
     }
   }
+  // Small grids: the whole-step kernel (its boundary work needs the fused plan above). The line lies where a step
+  // of the launch sequence costs as much (us per step, graph / whole-step kernel, one B200): Taylor-Green 64^3
+  // 110 / 101, 80^3 188 / 170, 88^3 212 / 245; channel with a sphere 32^3 102 / 57, 48^3 130 / 72, 80^3 255 / 198.
+  // A requested tile shape (ensemble members, the tuner, NSF_STAGE_TILE) means the streaming stage kernel.
+  constexpr size_t kStepMaxNodes = 550000;
+  if (!s->grouped && s->tileRequest < 0 && !std::getenv("NSF_STAGE_TILE") && L.bcBlocks > 0 && N <= kStepMaxNodes) {
+    const StepChoice ch = step_choose(G.NI, G.NJ, G.NK, s->nSM);
+    const StepShape t = step_shape(ch.shape);
+    const size_t smem = step_smem_bytes(ch.shape, ch.planes, L.bcLevels);
+    CK(cudaError_t(step_configure(ch.shape, smem)));
+    BcFlat fl;
+    bc_flatten({&s->bcLevels}, fl);
+    const int warps = int(std::min<long long>((fl.maxWork + 31) / 32, s->nSM));
+    const int blocks = std::min(std::max(ch.items, warps), step_capacity(ch.shape, smem, s->nSM));
+    if (blocks > 0) {
+      std::vector<StageItem> all, ordered;
+      for (int c0 = 1; c0 <= planes; c0 += ch.planes)
+        for (int j0 = 1; j0 <= G.NJ - 2; j0 += t.tj)
+          for (int k0 = 1; k0 <= G.NK - 2; k0 += t.tk)
+            all.push_back(StageItem{j0, k0, c0, std::min(planes, c0 + ch.planes - 1), 0});
+      std::vector<int> start(1, 0);
+      for (int b = 0; b < blocks; ++b) {
+        for (size_t q = size_t(b); q < all.size(); q += size_t(blocks)) ordered.push_back(all[q]);
+        start.push_back(int(ordered.size()));
+      }
+      if ((st = upload(s, &L.stepItems, ordered)) != NSF_OK) return st;
+      if ((st = upload(s, &L.stepStart, start)) != NSF_OK) return st;
+      if ((st = dalloc(s, &L.stepPart, 9 * size_t(blocks))) != NSF_OK) return st;
+      const std::vector<unsigned long long> zero(1, 0ull);
+      if ((st = upload(s, &L.stepSync, zero)) != NSF_OK) return st;
+      L.stepShape = ch.shape;
+      L.stepPlanes = ch.planes;
+      L.stepSmem = smem;
+      L.stepBlocks = blocks;
+    }
+  }
   if (S.bodiesInteract && L.bcBlocks == 0) {  // the separate boundary kernels treat all bodies at once
     s->err = "interacting immersed bodies need the fused boundary kernel, which this device cannot host";
     return NSF_ERR_GEOMETRY;
@@ -656,8 +692,22 @@ nsf_status build_device(nsf_solver* s) {
   // one step as a CUDA graph
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   s->launchesPerStep = enqueue_step(s->dGrid, G, L, s->stream);
+  if (L.stepBlocks > 0) s->launchesPerStep = 1;
   CK(cudaStreamEndCapture(s->stream, &s->graph));
   CK(cudaGraphInstantiate(&s->graphExec, s->graph, 0));
+  return NSF_OK;
+}
+
+// Queues nsteps steps on the handle's stream: the whole-step kernel where the grid has one (launches of at most
+// kStepsPerLaunch steps, so that other streams' work gets its turn), else one graph launch per step.
+constexpr uint64_t kStepsPerLaunch = 64;
+nsf_status queue_steps(nsf_solver* s, uint64_t nsteps) {
+  if (s->plan.stepBlocks > 0) {
+    for (uint64_t q = 0; q < nsteps; q += kStepsPerLaunch)
+      CK(cudaError_t(launch_steps(s->hGrid, s->dGrid, s->plan, int(std::min(kStepsPerLaunch, nsteps - q)), s->stream)));
+    return NSF_OK;
+  }
+  for (uint64_t q = 0; q < nsteps; ++q) CK(cudaGraphLaunch(s->graphExec, s->stream));
   return NSF_OK;
 }
 
@@ -752,8 +802,7 @@ nsf_status nsf_march(nsf_solver* s, uint64_t nsteps) {
     return NSF_ERR_STATE;
   }
   CK(cudaSetDevice(s->device));
-  for (uint64_t q = 0; q < nsteps; ++q) CK(cudaGraphLaunch(s->graphExec, s->stream));
-  return NSF_OK;
+  return queue_steps(s, nsteps);
 }
 
 // The control block after everything queued on the solver's stream: one copy into page-locked memory
@@ -1036,7 +1085,8 @@ nsf_status nsf_march_timed(nsf_solver* s, uint64_t nsteps, double* elapsed_ms) {
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
   CK(cudaEventRecord(a, s->stream));
-  for (uint64_t q = 0; q < nsteps; ++q) CK(cudaGraphLaunch(s->graphExec, s->stream));
+  const nsf_status st = queue_steps(s, nsteps);
+  if (st != NSF_OK) return st;
   CK(cudaEventRecord(b, s->stream));
   CK(cudaEventSynchronize(b));
   float ms = 0;

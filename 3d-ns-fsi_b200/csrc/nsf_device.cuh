@@ -226,10 +226,37 @@ struct LaunchPlan {
   int* bcItems;
   int* bcItemStart;
   unsigned long long* bcSync;  // device, 1 + 2 members counters, zero at creation
+  // Whole-step kernel (nsf_step.cu) of a small single grid: stepBlocks resident blocks run any number of steps
+  // in one launch. 0: a step is the launch sequence above, captured as a graph.
+  int stepBlocks;
+  int stepShape;   // StepTile
+  int stepPlanes;  // most planes of a tile
+  size_t stepSmem;
+  StageItem* stepItems;  // device; the tiles of block b are stepItems[stepStart[b] .. stepStart[b + 1])
+  int* stepStart;
+  double* stepPart;               // device, 9 x stepBlocks end-of-step partials
+  unsigned long long* stepSync;   // device, grid barrier counter, zero at creation
   int nSlots;
   bool hasBodies;
   bool hasFilter, hasGhostWork, hasSolid;
 };
+
+// Whole-step kernel (nsf_step.cu): tile shapes, the choice for a grid, and nsteps steps in one launch (returns a
+// cudaError_t). smem: dynamic shared memory of a block whose tiles have up to `planes` planes, with `levels`
+// levels of boundary work.
+enum StepTile { STEP_TILE_CUBE = 0, STEP_TILE_THIN = 1 };
+struct StepShape {
+  int tk, tj, maxPlanes, haloNodes;  // columns along k and j, most planes per tile, nodes of a staged plane
+};
+struct StepChoice {
+  int shape, planes, items;
+};
+StepShape step_shape(int shape);
+size_t step_smem_bytes(int shape, int planes, int levels);
+StepChoice step_choose(int NI, int NJ, int NK, int nSM);
+int step_configure(int shape, size_t smem);
+int step_capacity(int shape, size_t smem, int nSM);
+int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream);
 
 // Host entry points of nsf_kernels.cu.
 // Stage-kernel variant queries (v: StageTile).
