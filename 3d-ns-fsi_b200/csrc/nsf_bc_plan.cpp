@@ -288,4 +288,31 @@ std::vector<int> bc_block_ranges(const BcFlat& fl, int capacity) {
   return start;
 }
 
+void mark_filter_planes(const Grid& G, const std::vector<long long>& fnode, int tj, int tk, int g,
+                        std::vector<StageItem>& items) {
+  const int nj = (G.NJ - 2 + tj - 1) / tj, nk = (G.NK - 2 + tk - 1) / tk;
+  std::vector<uint8_t> has(size_t(nj) * nk * G.NI, 0);  // [tile][plane]
+  // tiles t of w columns whose staged columns t * w .. (t + 1) * w + 1 hold index c
+  auto range = [](int c, int w, int n, int& lo, int& hi) {
+    lo = c < 2 ? 0 : (c - 2) / w;
+    hi = std::min(n - 1, c / w);
+  };
+  for (long long n : fnode) {
+    const int i = int(n / G.sI), j = int(n % G.sI / G.sJ), k = int(n % G.sJ);
+    int j0, j1, k0, k1;
+    range(j, tj, nj, j0, j1);
+    range(k, tk, nk, k0, k1);
+    for (int a = j0; a <= j1; ++a)
+      for (int b = k0; b <= k1; ++b) has[(size_t(a) * nk + b) * G.NI + i] = 1;
+  }
+  for (StageItem& w : items) {
+    if (w.g != g) continue;
+    const uint8_t* h = has.data() + (size_t((w.j0 - 1) / tj) * nk + (w.k0 - 1) / tk) * G.NI;
+    w.f0 = w.i0 - 1;
+    w.f1 = w.i1 + 1;
+    while (w.f0 <= w.f1 && !h[w.f0]) ++w.f0;
+    while (w.f1 >= w.f0 && !h[w.f1]) --w.f1;
+  }
+}
+
 }  // namespace nsf

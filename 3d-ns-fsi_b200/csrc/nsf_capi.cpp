@@ -559,6 +559,8 @@ nsf_status build_device(nsf_solver* s) {
     for (int tj = 0; tj < nj; ++tj)
       for (int tk = 0; tk < nk; ++tk)
         items.push_back(StageItem{1 + tj * TJ, 1 + tk * TK, c0, std::min(planes, c0 + clen - 1), 0});
+  mark_filter_planes(G, fnode, TJ, TK, 0, items);
+  s->filterNodes = fnode;
   L.nItems = int(items.size());
   L.stageBlocks = std::min(L.nItems, slots);
   {  // CTA b takes items b, b + stageBlocks, ... (whole waves of equal items), stored contiguously

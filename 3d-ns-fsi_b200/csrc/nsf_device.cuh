@@ -142,6 +142,9 @@ enum StageTile { STAGE_TILE_32x8 = 0, STAGE_TILE_16x16 = 1 };
 struct StageItem {
   int j0, k0, i0, i1;  // tile origin (first computed j, k) and inclusive i range
   int g;               // ensemble member (0 for a single grid)
+  // staged planes that may hold near-body filter nodes within the tile and its halo, inclusive (mark_filter_planes;
+  // the default is every plane)
+  int f0 = 0, f1 = 1 << 30;
 };
 
 // Launch geometry of one step, fixed at initialisation.
@@ -319,6 +322,10 @@ void bc_flatten(const std::vector<const BcMemberLevels*>& members, BcFlat& out);
 // the members' work (at least one each, never more than a member can use); returns the members + 1 range
 // starts, empty if the members do not fit.
 std::vector<int> bc_block_ranges(const BcFlat& fl, int capacity);
+// Narrows f0 .. f1 of member g's items to the planes where one of the filter nodes (device indices) lies in the
+// item's tile of tj x tk columns or its one-node halo (nsf_bc_plan.cpp).
+void mark_filter_planes(const Grid& G, const std::vector<long long>& fnode, int tj, int tk, int g,
+                        std::vector<StageItem>& items);
 // The node a periodic face node finally copies (opposite interior plane, then further periodic faces).
 void periodic_source_host(const Grid& G, int axis, int side, int ijk[3]);
 void launch_ghost_weights(int nGhost, const double* pts, const double* nrm, const uint8_t* flags, const double* ipl,

@@ -254,6 +254,8 @@ nsf_status build_ensemble(nsf_ensemble* e, const char* cache) {
     }
   }
   (void)bestLen;
+  for (int g = 0; g < M; ++g)
+    mark_filter_planes(e->members[g]->hGrid, e->members[g]->filterNodes, TJ, TK, g, ordered);
   L.nItems = int(ordered.size());
   L.stageBlocks = int(start.size()) - 1;
   nsf_status st;

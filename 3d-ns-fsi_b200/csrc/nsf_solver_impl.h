@@ -49,6 +49,7 @@ struct nsf_solver {
   // node flags to add (EDGE_PLANE_BIT on halo planes and on the whole grid's edge planes); empty otherwise
   std::vector<double> slabCons, slabPrim;
   std::vector<uint8_t> slabFlags;
+  std::vector<long long> filterNodes;  // device node of each near-body filter slot
   std::vector<int> ghostOrder;   // device ghost slot -> position in the bodies' ghost lists
   nsf::BcMemberLevels bcLevels;  // dependency levels of the boundary work (fused boundary kernel)
   nsf::StepCtl ctlInit{};  // the control block at level 0 (the discrete adjoint restarts from it)

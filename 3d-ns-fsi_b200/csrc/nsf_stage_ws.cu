@@ -17,8 +17,8 @@
 //     see x_node / x_face in nsf_physics.cuh) and carries them in registers along the column; the
 //     RHS of the previous plane is then G/F differences plus the y/z terms read from the staged planes,
 //     and the RK4 combine is written with coalesced 256-byte row stores.
-// Warpgroup 0 runs with 88 registers per thread and the column warpgroups with 208 (setmaxnreg), so
-// the register-hungry RHS does not spill while the CTA still has twelve warps.
+// Warpgroup 0 runs with 88 registers per thread and the column warpgroups with 208 (setmaxnreg; 104 and 200 with
+// filter nodes), so the register-hungry RHS does not spill while the CTA still has twelve warps.
 //
 // Ring slots have a "full" and an "empty" mbarrier. Every wait is bounded: a wait that gives up sets
 // StepCtl::timeout and a CTA-wide abort flag that ends every other wait at once; the producer then
@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "nsf_device.cuh"
 #include "nsf_internal.h"
@@ -40,16 +41,17 @@
 namespace nsf {
 namespace ws {
 constexpr int NSTAGE = 96;                        // staging threads (warps 1-3)
+constexpr int NPASS = 4;                          // staged nodes per staging thread and plane
 constexpr int NC = 5, NP = 5, NE = 3;             // conserved / primitive / epilogue ring depths
 constexpr int NPRIM = 6;                          // staged primitive fields: u, v, w, p, T, mu (kappa = pf mu)
 constexpr int MAP_CONS = 0, MAP_EPI = 15, MAP_ACC = 30, MAP_TYPE = 35, NMAPS = 36;
 constexpr long long WAIT_LIMIT = 1ll << 22;  // default polls before a wait is declared failed (StepCtl::waitLimit)
-// Register split (setmaxnreg): the launch gives every thread 168 registers (384 x 168 = 64,512); the
-// split must not exceed that total: 128 x 88 + 256 x 208 = 64,512.
-constexpr int REG_LAUNCH = 168, REG_LOW = 88, REG_HIGH = 208;
-// The ensemble's stage-4 instantiation (per-item coefficients and the dt / norm accumulators) gives its
-// column threads 8 more: 128 x 72 + 256 x 216 = 64,512.
-constexpr int REG_LOW_ENS4 = 72, REG_HIGH_ENS4 = 216;
+// Register split (setmaxnreg): the launch gives every thread 168 registers (384 x 168 = 64,512); a split must not
+// exceed that total. Warpgroup 0 gets 88 and the column warpgroups 208: 128 x 88 + 256 x 208 = 64,512. With
+// near-body filter nodes (FLT) the staging of a body's planes needs more, 128 x 104 + 256 x 200 = 64,512 (sphere
+// 128^3: 485 us per step against 494 with 88 / 208); an ensemble's stage 4 stays at 88 / 208, since its columns
+// spill below (64 members: 3990 us per step, 4003 with 104 / 200, 4047 with 72 / 216).
+constexpr int REG_LAUNCH = 168, REG_LOW = 88, REG_HIGH = 208, REG_LOW_FLT = 104, REG_HIGH_FLT = 200;
 
 constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -98,9 +100,9 @@ struct Tile {
   static_assert(OFF_PRIM % 128 == 0 && OFF_EPI % 128 == 0 && CONS_SLOT % 128 == 0 && TYPE_OFF % 128 == 0,
                 "TMA destinations need 128 B alignment");
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
-  static_assert(NSTAGE * 4 >= HP, "four staging passes cover a plane");
+  static_assert(NSTAGE * NPASS >= HP && NSTAGE * (NPASS - 1) <= HP && NPASS % 2 == 0, "four staging passes cover a plane");
   static_assert(128 * REG_LOW + NCOL * REG_HIGH <= NTHREADS * REG_LAUNCH, "register split exceeds the launch total");
-  static_assert(128 * REG_LOW_ENS4 + NCOL * REG_HIGH_ENS4 <= NTHREADS * REG_LAUNCH, "register split exceeds the launch total");
+  static_assert(128 * REG_LOW_FLT + NCOL * REG_HIGH_FLT <= NTHREADS * REG_LAUNCH, "register split exceeds the launch total");
 };
 }  // namespace ws
 
@@ -165,7 +167,12 @@ __device__ __forceinline__ void reg_alloc() {
 // only stage with dt maxima, change norms and the NaN check; mode 1 carries none of their registers). The
 // single grid runs mode 0 for stages 1-3 and mode 2 for stage 4, an ensemble modes 1 and 2: the fastest
 // pairing measured (mode 1 frees registers an ensemble needs, but its schedule is slower for one grid).
-template <int TK_, int TJ_, bool ENS, int MODE>
+// FLT: the grid has near-body filter nodes. Without them the staging looks at no node type; with them it takes an
+// item that has any (StageItem::f0 .. f1) through a second copy of its loop. The staging warps pace the kernel: in
+// one loop for both, a pair of filter nodes held their warp up for four trips to L2 in a row, and any work added
+// for it slowed every grid by 5-7 %. Measured (us per step, before / now): sphere 96^3 379 / 293, sphere 128^3
+// 579 / 485, 16 spheres 256x128x128 980 / 866, the 64-member ensemble 4069 / 3990, Taylor-Green 128^3 440 / 431.
+template <int TK_, int TJ_, bool ENS, int MODE, bool FLT>
 __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
     k_stage_ws(const __grid_constant__ Grid G0, const Grid* __restrict__ grids, const StageItem* __restrict__ items,
                const int* __restrict__ ctaStart, int s) {
@@ -238,7 +245,7 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
   auto skip = [&](const StageItem& w) { return ENS && !ctl_of(grid_of(w)).active; };
 
   if (warp < 4) {
-    reg_dealloc<(ENS && MODE == 2) ? REG_LOW_ENS4 : REG_LOW>();
+    reg_dealloc<FLT && !(ENS && MODE == 2) ? REG_LOW_FLT : REG_LOW>();
     if (warp == 0) {
       // ------------------------------------------------------------------ producer (one thread)
       if (lane == 0) {
@@ -344,60 +351,95 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
         const Grid& G = grid_of(w);
         const ThermoConsts C{G.C.gamma, G.C.gm1, G.C.sc1, G.C.re, G.C.pf};
         const double* __restrict__ fpre = G.fpre;
+        const int* const fidx = G.fidx;
         const long long sIs = G.sI, sJs = G.sJ;
-        for (int p = w.i0 - 1; p <= w.i1 + 1; ++p, ++q) {
-          const uint32_t sl = q % NC, ps = q % NP;
-          if (q >= NP) ok = mbar_wait(&primEmpty[ps], ((q / NP) - 1) & 1, abortFlag, lim);
-          ok = ok && mbar_wait(&consFull[sl], (q / NC) & 1, abortFlag, lim);
-          if (!ok) {
-            fail(G);
-            break;
-          }
-          const double* cs = reinterpret_cast<const double*>(sm + OFF_CONS + sl * CONS_SLOT);
-          const uint8_t* ts = reinterpret_cast<const uint8_t*>(cs) + TYPE_OFF;
-          double* pv = reinterpret_cast<double*>(sm + OFF_PRIM + ps * PRIM_SLOT);
-          // Two nodes per pass (idx and idx + NSTAGE) so that their long dependency chains (reciprocal,
-          // square root, division) overlap. Nodes past the mesh read TMA zero fill: finite values that
-          // are never used. Slots past the plane (idx >= HP) compute a dummy node and store nothing.
-#pragma unroll 1
-          for (int idx = st; idx < HP; idx += 2 * NSTAGE) {
-            const int idy = idx + NSTAGE, idyc = idy < HP ? idy : idx;
-            double rho[2] = {cs[0 * FS + idx], cs[0 * FS + idyc]}, rE[2] = {cs[4 * FS + idx], cs[4 * FS + idyc]};
+        auto store = [&](double* pv, int idx, const Prim& a) {
+          pv[0 * FS + idx] = a.u;
+          pv[1 * FS + idx] = a.v;
+          pv[2 * FS + idx] = a.w;
+          pv[3 * FS + idx] = a.p;
+          pv[4 * FS + idx] = a.T;
+          pv[5 * FS + idx] = a.mu;
+        };
+        // One item's planes; BODY: an item with filter nodes in some of its staged planes (f0 .. f1).
+        auto stage_planes = [&](auto body) {
+          constexpr bool BODY = decltype(body)::value;
+          int slot[NPASS];  // filter slots of this thread's nodes (st + NSTAGE m) in the coming plane, -1: none
+          auto slots_of = [&](int p) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int id = h ? idyc : idx;
-              const int hj = id / HK, hk = id - hj * HK;
-              if (ts[hj * TYW + hk] & FILTER_BIT) {
-                const long long n = (long long)p * sIs + (long long)(w.j0 - 1 + hj) * sJs + (w.k0 - 1 + hk);
-                const int f = __ldg(G.fidx + n);
-                rho[h] = fpre[2 * f];
-                rE[h] = fpre[2 * f + 1];
+            for (int m = 0; m < NPASS; ++m) {
+              const int id = st + NSTAGE * m, hj = id / HK, hk = id - hj * HK;
+              const int j = w.j0 - 1 + hj, k = w.k0 - 1 + hk;
+              slot[m] = id < HP && j < G.NJ && k < G.NK ? __ldg(fidx + p * sIs + j * sJs + k) : -1;
+            }
+          };
+          if (BODY && w.i0 - 1 >= w.f0) slots_of(w.i0 - 1);
+          for (int p = w.i0 - 1; p <= w.i1 + 1; ++p, ++q) {
+            const uint32_t sl = q % NC, ps = q % NP;
+            const double* cs = reinterpret_cast<const double*>(sm + OFF_CONS + sl * CONS_SLOT);
+            double* pv = reinterpret_cast<double*>(sm + OFF_PRIM + ps * PRIM_SLOT);
+            const bool here = BODY && p >= w.f0 && p <= w.f1;
+            // A filter node's values take two trips to L2, one after the other: its slot, then the slot's pre-filter
+            // rho and rho_E. The slots are read while the plane before is staged; the values come into L1 while the
+            // plane is waited for.
+            int cur[NPASS] = {-1, -1, -1, -1};
+            if (here) {
+#pragma unroll
+              for (int m = 0; m < NPASS; ++m) {
+                cur[m] = slot[m];
+                if (cur[m] >= 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(fpre + 2 * cur[m]));
               }
             }
-            const Prim a0 = prims_of_nr(C, rho[0], cs[1 * FS + idx], cs[2 * FS + idx], cs[3 * FS + idx], rE[0]);
-            const Prim a1 = prims_of_nr(C, rho[1], cs[1 * FS + idyc], cs[2 * FS + idyc], cs[3 * FS + idyc], rE[1]);
-            pv[0 * FS + idx] = a0.u;
-            pv[1 * FS + idx] = a0.v;
-            pv[2 * FS + idx] = a0.w;
-            pv[3 * FS + idx] = a0.p;
-            pv[4 * FS + idx] = a0.T;
-            pv[5 * FS + idx] = a0.mu;
-            if (idy < HP) {
-              pv[0 * FS + idy] = a1.u;
-              pv[1 * FS + idy] = a1.v;
-              pv[2 * FS + idy] = a1.w;
-              pv[3 * FS + idy] = a1.p;
-              pv[4 * FS + idy] = a1.T;
-              pv[5 * FS + idy] = a1.mu;
+            if (BODY && p + 1 >= w.f0 && p + 1 <= w.f1 && p <= w.i1) slots_of(p + 1);  // the last plane is i1 + 1
+            if (q >= NP) ok = mbar_wait(&primEmpty[ps], ((q / NP) - 1) & 1, abortFlag, lim);
+            ok = ok && mbar_wait(&consFull[sl], (q / NC) & 1, abortFlag, lim);
+            if (!ok) {
+              fail(G);
+              break;
             }
+            // Two nodes per pass (idx and idx + NSTAGE) so that their long dependency chains (reciprocal,
+            // square root, division) overlap. Nodes past the mesh read TMA zero fill: finite values that
+            // are never used. Slots past the plane (idx >= HP) compute a dummy node and store nothing.
+            if (here) {
+#pragma unroll
+              for (int m = 0; m < NPASS; m += 2) {
+                const int idx = st + NSTAGE * m, idy = idx + NSTAGE, idyc = idy < HP ? idy : idx;  // idx < HP
+                double rho[2] = {cs[0 * FS + idx], cs[0 * FS + idyc]}, rE[2] = {cs[4 * FS + idx], cs[4 * FS + idyc]};
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                  if (cur[m + h] >= 0) {
+                    rho[h] = fpre[2 * cur[m + h]];
+                    rE[h] = fpre[2 * cur[m + h] + 1];
+                  }
+                const Prim a0 = prims_of_nr(C, rho[0], cs[1 * FS + idx], cs[2 * FS + idx], cs[3 * FS + idx], rE[0]);
+                const Prim a1 = prims_of_nr(C, rho[1], cs[1 * FS + idyc], cs[2 * FS + idyc], cs[3 * FS + idyc], rE[1]);
+                store(pv, idx, a0);
+                if (idy < HP) store(pv, idy, a1);
+              }
+            } else {
+#pragma unroll 1
+              for (int idx = st; idx < HP; idx += 2 * NSTAGE) {
+                const int idy = idx + NSTAGE, idyc = idy < HP ? idy : idx;
+                const Prim a0 = prims_of_nr(C, cs[0 * FS + idx], cs[1 * FS + idx], cs[2 * FS + idx], cs[3 * FS + idx],
+                                            cs[4 * FS + idx]);
+                const Prim a1 = prims_of_nr(C, cs[0 * FS + idyc], cs[1 * FS + idyc], cs[2 * FS + idyc],
+                                            cs[3 * FS + idyc], cs[4 * FS + idyc]);
+                store(pv, idx, a0);
+                if (idy < HP) store(pv, idy, a1);
+              }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&primFull[ps]);
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&primFull[ps]);
-        }
+        };
+        if (FLT && G.nFilter > 0 && w.f0 <= w.f1)
+          stage_planes(std::true_type{});
+        else
+          stage_planes(std::false_type{});
       }
     }
   } else {
-    reg_alloc<(ENS && MODE == 2) ? REG_HIGH_ENS4 : REG_HIGH>();
+    reg_alloc<FLT && !(ENS && MODE == 2) ? REG_HIGH_FLT : REG_HIGH>();
     // -------------------------------------------------------------------- columns (warpgroups 1-2)
     const int ct = tid - 128, tx = ct % TK, ty = ct / TK;
     const int cidx = (ty + 1) * HK + (tx + 1);   // this column's node in a staged plane
@@ -671,8 +713,9 @@ namespace {
 struct VariantInfo {
   int tk, tj, threads, typeBoxW;
   size_t smem;
-  const void* fn[2];     // single grid: stages 1-3 (mode 0), stage 4 (mode 2)
-  const void* fnEns[2];  // ensemble: stages 1-3 (mode 1), stage 4 (mode 2)
+  // single grid: stages 1-3 (mode 0), stage 4 (mode 2); the same with near-body filter nodes; an ensemble's stages
+  // 1-3 (mode 1), stage 4 (mode 2)
+  const void* fn[6];
 };
 template <int TK, int TJ>
 VariantInfo variant_info() {
@@ -682,10 +725,12 @@ VariantInfo variant_info() {
                      TL::NTHREADS,
                      TL::TYW,
                      TL::SMEM,
-                     {reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 0>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 2>)},
-                     {reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 1>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 2>)}};
+                     {reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 0, false>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 2, false>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 0, true>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 2, true>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 1, true>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 2, true>)}};
 }
 VariantInfo info(int v) { return v == STAGE_TILE_16x16 ? variant_info<16, 16>() : variant_info<32, 8>(); }
 
@@ -693,10 +738,18 @@ template <int TK, int TJ, bool ENS>
 void launch_variant(const Grid& hg, const Grid* dGrids, const LaunchPlan& L, int s, cudaStream_t st) {
   using TL = ws::Tile<TK, TJ>;
   constexpr int early = ENS ? 1 : 0;  // the instantiation of stages 1-3
-  if (s == 3)
-    k_stage_ws<TK, TJ, ENS, 2><<<L.stageBlocks, TL::NTHREADS, TL::SMEM, st>>>(hg, dGrids, L.items, L.ctaStart, s);
+  auto go = [&](auto kernel) {
+    kernel<<<L.stageBlocks, TL::NTHREADS, TL::SMEM, st>>>(hg, dGrids, L.items, L.ctaStart, s);
+  };
+  constexpr bool plain = ENS;  // a grid without filter nodes runs FLT = ENS
+  if (L.hasFilter && s == 3)
+    go(k_stage_ws<TK, TJ, ENS, 2, true>);
+  else if (L.hasFilter)
+    go(k_stage_ws<TK, TJ, ENS, early, true>);
+  else if (s == 3)
+    go(k_stage_ws<TK, TJ, ENS, 2, plain>);
   else
-    k_stage_ws<TK, TJ, ENS, early><<<L.stageBlocks, TL::NTHREADS, TL::SMEM, st>>>(hg, dGrids, L.items, L.ctaStart, s);
+    go(k_stage_ws<TK, TJ, ENS, early, plain>);
 }
 }  // namespace
 
@@ -704,7 +757,7 @@ size_t stage_smem_bytes(int v) { return info(v).smem; }
 int stage_configure(int v) {
   const VariantInfo vi = info(v);
   cudaError_t e = cudaSuccess;
-  for (const void* fn : {vi.fn[0], vi.fn[1], vi.fnEns[0], vi.fnEns[1]})
+  for (const void* fn : vi.fn)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(vi.smem));
   return int(e);
 }
@@ -724,7 +777,7 @@ int stage_num_maps() { return ws::NMAPS; }
 int stage_launch_registers(int v) {
   const VariantInfo vi = info(v);
   int r = 1 << 30;
-  for (const void* fn : {vi.fn[0], vi.fn[1], vi.fnEns[0], vi.fnEns[1]}) {
+  for (const void* fn : vi.fn) {
     cudaFuncAttributes a{};
     if (cudaFuncGetAttributes(&a, fn) != cudaSuccess) return -1;
     r = a.numRegs < r ? a.numRegs : r;
@@ -733,7 +786,7 @@ int stage_launch_registers(int v) {
 }
 bool stage_register_split_ok(int v) {
   const int r = stage_launch_registers(v);
-  const int need = std::max(128 * ws::REG_LOW + 256 * ws::REG_HIGH, 128 * ws::REG_LOW_ENS4 + 256 * ws::REG_HIGH_ENS4);
+  const int need = std::max(128 * ws::REG_LOW + 256 * ws::REG_HIGH, 128 * ws::REG_LOW_FLT + 256 * ws::REG_HIGH_FLT);
   return r > 0 && need <= info(v).threads * r;
 }
 void launch_stage(const Grid& hg, const LaunchPlan& L, int s, void* stream) {

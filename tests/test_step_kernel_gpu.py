@@ -65,6 +65,22 @@ def test_equals_the_launch_sequence(flow, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tile", ["32x8", "16x16"])
+@pytest.mark.parametrize("flow,n", [("sphere", (40, 47, 45)), ("walls", (37, 39, 50)), ("shipped", (61, 33, 3))],
+                         ids=["sphere", "walls", "shipped"])
+def test_streaming_kernel_with_bodies(flow, n, tile, monkeypatch):
+    """The streaming kernel's staging of body planes, per tile shape: bodies that lie across tile edges."""
+    cfg = config(flow, n, 9, filt=3)
+    with nsfsi.Solver(cfg) as s:
+        monkeypatch.setenv("NSF_STAGE_TILE", tile)
+        with nsfsi.Solver(cfg) as g:
+            assert s.launches_per_step() == 1 < g.launches_per_step()
+            s.march(9)
+            g.march(9)
+            assert_same(s, g)
+
+
+@pytest.mark.gpu
 def test_many_steps_and_the_end_time_stop():
     """More steps than one launch takes, and steps past t_end, which are no-ops."""
     cfg = config("sphere", (30, 29, 31), 200, end_time=0.5)
