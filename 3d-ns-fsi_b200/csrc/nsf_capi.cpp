@@ -807,11 +807,15 @@ nsf_status nsf_march(nsf_solver* s, uint64_t nsteps) {
   return queue_steps(s, nsteps);
 }
 
-// The control block after everything queued on the solver's stream: one copy into page-locked memory
-// queued behind that work, then one wait.
+// The control block after everything queued on the solver's stream: written into page-locked host memory by a
+// kernel queued behind that work, then one wait. (A copy would queue on the device's download engine behind a
+// snapshot still travelling to the host: 805 MB, 16 ms, for the 256^3 Taylor-Green case's saved fields.)
 static nsf_status read_ctl(nsf_solver* s, StepCtl* out) {
-  if (!s->hCtl) CK(cudaMallocHost(&s->hCtl, sizeof(StepCtl)));
-  CK(cudaMemcpyAsync(s->hCtl, s->dCtl, sizeof(StepCtl), cudaMemcpyDeviceToHost, s->stream));
+  if (!s->hCtl) CK(cudaHostAlloc(&s->hCtl, sizeof(StepCtl), cudaHostAllocMapped));
+  void* dev = nullptr;
+  CK(cudaHostGetDevicePointer(&dev, s->hCtl, 0));
+  launch_ctl_out(s->dCtl, static_cast<StepCtl*>(dev), s->stream);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s->stream));
   *out = *s->hCtl;
   return NSF_OK;

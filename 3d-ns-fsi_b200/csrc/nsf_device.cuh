@@ -346,6 +346,8 @@ struct SnapInactive {
   const double* p7Ic;
   int countIc;
 };
+// Queues a copy of the control block into `out` (device address of page-locked host memory) by a kernel.
+void launch_ctl_out(const StepCtl* ctl, StepCtl* out, void* stream);
 // Queues the snapshot of the slots' fields into `out` (packed, NI*NJ*NK doubles per slot) on `stream`.
 void launch_snapshot(const Grid* dg, const SnapSlots& sl, const SnapInactive& in, double* out, int nSM, void* stream);
 

@@ -566,6 +566,16 @@ void launch_ghost_weights(int nGhost, const double* pts, const double* nrm, cons
   if (nGhost > 0) k_ghost_weights<<<(nGhost + 127) / 128, 128, 0, st>>>(nGhost, pts, nrm, flags, ipl, dx, dy, dz, w);
 }
 
+__global__ void k_ctl_out(const StepCtl* __restrict__ ctl, StepCtl* __restrict__ out) {
+  const unsigned long long* a = reinterpret_cast<const unsigned long long*>(ctl);
+  unsigned long long* b = reinterpret_cast<unsigned long long*>(out);
+  for (int q = threadIdx.x; q < int(sizeof(StepCtl) / 8); q += blockDim.x) b[q] = a[q];
+}
+
+void launch_ctl_out(const StepCtl* ctl, StepCtl* out, void* stream) {
+  k_ctl_out<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(ctl, out);
+}
+
 void launch_snapshot(const Grid* dg, const SnapSlots& sl, const SnapInactive& in, double* out, int nSM, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   k_snapshot<<<nSM * 8, 256, 0, st>>>(dg, sl, out);
