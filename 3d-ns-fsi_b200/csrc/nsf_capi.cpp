@@ -572,6 +572,11 @@ nsf_status build_device(nsf_solver* s) {
     }
     items.swap(ordered);
     if ((st = upload(s, &L.ctaStart, start)) != NSF_OK) return st;
+    for (int b = 0; b < L.stageBlocks; ++b) {
+      int span = 0;
+      for (int q = start[b]; q < start[b + 1]; ++q) span += items[q].i1 - items[q].i0 + 3;
+      L.stageSpan = std::max(L.stageSpan, span);
+    }
   }
   if ((st = upload(s, &L.items, items)) != NSF_OK) return st;
   std::vector<EdgeBlock> ebAxis[3];
@@ -737,6 +742,53 @@ double nsf_initial_dt(const nsf_config& c, const nsf::HostSetup& S, const std::v
   return initial_dt(c, S, cons, prim);
 }
 
+// The control block after everything queued on the solver's stream: written into page-locked host memory by a
+// kernel queued behind that work, then one wait. (A copy would queue on the device's download engine behind a
+// snapshot still travelling to the host: 805 MB, 16 ms, for the 256^3 Taylor-Green case's saved fields.)
+static nsf_status read_ctl(nsf_solver* s, StepCtl* out) {
+  if (!s->hCtl) CK(cudaHostAlloc(&s->hCtl, sizeof(StepCtl), cudaHostAllocMapped));
+  void* dev = nullptr;
+  CK(cudaHostGetDevicePointer(&dev, s->hCtl, 0));
+  launch_ctl_out(s->dCtl, static_cast<StepCtl*>(dev), s->stream);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(s->stream));
+  *out = *s->hCtl;
+  return NSF_OK;
+}
+
+nsf_status nsf_download_planes(nsf_solver* s, uint32_t mask, size_t first, size_t count, double* host, size_t pitch) {
+  int nf = 0;
+  const SnapSlots sl = snap_slots(mask, &nf);
+  if (!nf) return NSF_OK;
+  CK(cudaSetDevice(s->device));
+  const HostSetup& S = s->setup;
+  const size_t plane = S.NJ * S.NK;
+  if ((mask & ~0x1Fu) == 0) {  // conserved fields only: copied straight from their current buffers
+    StepCtl ctl;
+    const nsf_status st = read_ctl(s, &ctl);
+    if (st != NSF_OK) return st;
+    const size_t hp = S.NK * sizeof(double), dp = size_t(s->hGrid.NKp) * sizeof(double);
+    for (int f = 0; f < 5; ++f)
+      if (sl.slot[f] >= 0)
+        CK(cudaMemcpy2DAsync(host + size_t(sl.slot[f]) * pitch, hp,
+                             s->hGrid.bufs[ctl.perm[f][0]][f] + first * size_t(s->hGrid.sI), dp, hp, count * S.NJ,
+                             cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    return NSF_OK;
+  }
+  double* tmp = nullptr;
+  CK(cudaMalloc(&tmp, size_t(nf) * S.N * sizeof(double)));
+  launch_snapshot(s->dGrid, sl, snap_inactive(s), tmp, s->nSM, s->stream);
+  cudaError_t e = cudaGetLastError();
+  for (int q = 0; q < nf && e == cudaSuccess; ++q)
+    e = cudaMemcpyAsync(host + size_t(q) * pitch, tmp + size_t(q) * S.N + first * plane, count * plane * sizeof(double),
+                        cudaMemcpyDeviceToHost, s->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+  cudaFree(tmp);
+  if (e != cudaSuccess) return cuda_fail(s, e, "download");
+  return NSF_OK;
+}
+
 extern "C" {
 
 nsf_status nsf_create(const nsf_config* cfg, int32_t device, nsf_solver** out) {
@@ -807,20 +859,6 @@ nsf_status nsf_march(nsf_solver* s, uint64_t nsteps) {
   return queue_steps(s, nsteps);
 }
 
-// The control block after everything queued on the solver's stream: written into page-locked host memory by a
-// kernel queued behind that work, then one wait. (A copy would queue on the device's download engine behind a
-// snapshot still travelling to the host: 805 MB, 16 ms, for the 256^3 Taylor-Green case's saved fields.)
-static nsf_status read_ctl(nsf_solver* s, StepCtl* out) {
-  if (!s->hCtl) CK(cudaHostAlloc(&s->hCtl, sizeof(StepCtl), cudaHostAllocMapped));
-  void* dev = nullptr;
-  CK(cudaHostGetDevicePointer(&dev, s->hCtl, 0));
-  launch_ctl_out(s->dCtl, static_cast<StepCtl*>(dev), s->stream);
-  CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(s->stream));
-  *out = *s->hCtl;
-  return NSF_OK;
-}
-
 nsf_status nsf_sync(nsf_solver* s) {
   if (!s || !s->initialized || s->hostOnly) return s ? NSF_ERR_STATE : NSF_ERR_ARG;
   StepCtl ctl;
@@ -871,33 +909,7 @@ nsf_status nsf_get_time(nsf_solver* s, double* t, uint64_t* level, double* dt) {
 nsf_status nsf_download(nsf_solver* s, uint32_t mask, double* host) {
   if (!s || !host) return NSF_ERR_ARG;
   if (!s->initialized || s->hostOnly) return NSF_ERR_STATE;
-  int nf = 0;
-  const SnapSlots sl = snap_slots(mask, &nf);
-  if (!nf) return NSF_OK;
-  CK(cudaSetDevice(s->device));
-  if ((mask & ~0x1Fu) == 0) {  // conserved fields only: copied straight from their current buffers
-    StepCtl ctl;
-    const nsf_status st = read_ctl(s, &ctl);
-    if (st != NSF_OK) return st;
-    const HostSetup& S = s->setup;
-    const size_t hp = S.NK * sizeof(double), dp = size_t(s->hGrid.NKp) * sizeof(double);
-    for (int f = 0; f < 5; ++f)
-      if (sl.slot[f] >= 0)
-        CK(cudaMemcpy2DAsync(host + size_t(sl.slot[f]) * S.N, hp, s->hGrid.bufs[ctl.perm[f][0]][f], dp, hp,
-                             S.NI * S.NJ, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-    return NSF_OK;
-  }
-  const size_t bytes = size_t(nf) * s->setup.N * sizeof(double);
-  double* tmp = nullptr;
-  CK(cudaMalloc(&tmp, bytes));
-  launch_snapshot(s->dGrid, sl, snap_inactive(s), tmp, s->nSM, s->stream);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(host, tmp, bytes, cudaMemcpyDeviceToHost, s->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-  cudaFree(tmp);
-  if (e != cudaSuccess) return cuda_fail(s, e, "download");
-  return NSF_OK;
+  return nsf_download_planes(s, mask, 0, s->setup.NI, host, s->setup.N);
 }
 
 nsf_status nsf_download_async(nsf_solver* s, uint32_t mask, double* host, uint64_t* ticket) {

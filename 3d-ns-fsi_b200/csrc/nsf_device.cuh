@@ -211,6 +211,7 @@ struct LaunchPlan {
   int nSM;
   int tile;  // StageTile
   int stageBlocks;
+  int stageSpan;  // planes the busiest block streams in a stage launch (its items' planes and two halo planes each)
   int nItems;
   StageItem* items;  // device; the items of CTA b are items[ctaStart[b] .. ctaStart[b + 1])
   int* ctaStart;     // device, stageBlocks + 1 entries
@@ -281,10 +282,10 @@ void launch_stage_ensemble(const Grid* dGrids, const LaunchPlan& L, int s, void*
 // value to the stage kernel, whose coefficients then come from the constant bank).
 int enqueue_step(Grid* dg, const Grid& hg, const LaunchPlan& L, void* stream);
 // Pieces of a step for callers that put work between them (x-slab groups, nsf_slab.cpp): the prologue and
-// the density filter of one grid; the fused boundary kernel of stage s (fin: with the end-of-step finalize).
-// Return the launches queued.
-int enqueue_step_begin(Grid* dg, const LaunchPlan& L, void* stream);
-int launch_bc_part(Grid* dg, const LaunchPlan& L, int s, bool fin, void* stream);
+// the density filter of several grids (dg: their device array); the fused boundary kernel of stage s (fin: with the
+// end-of-step finalize). Return the launches queued.
+int enqueue_step_begin(Grid* dg, int members, const LaunchPlan& L, void* stream);
+int launch_bc_part(Grid* dg, int members, const LaunchPlan& L, int s, bool fin, void* stream);
 // Same sequence with events recorded around each of the four stage kernels (events[2*s], events[2*s+1]);
 // used for per-kernel timing. inGraph: the stream is being captured, and the events become event-record
 // nodes of the graph (so the kernels are timed inside graph replays, as the solver runs them).

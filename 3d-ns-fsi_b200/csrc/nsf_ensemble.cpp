@@ -44,20 +44,15 @@ struct nsf_ensemble {
 
 namespace {
 
-#define CKE(call)                                                          \
-  do {                                                                     \
-    cudaError_t e_ = (call);                                               \
-    if (e_ != cudaSuccess) {                                               \
-      e->err = std::string(#call) + ": " + cudaGetErrorString(e_);         \
-      return NSF_ERR_CUDA;                                                 \
-    }                                                                      \
-  } while (0)
-
 template <class T>
-nsf_status ens_alloc(nsf_ensemble* e, T** p, size_t count) {
+nsf_status group_alloc(std::vector<void*>& allocs, std::string& err, T** p, size_t count) {
   void* q = nullptr;
-  CKE(cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
-  e->allocs.push_back(q);
+  const cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
+  if (e != cudaSuccess) {
+    err = std::string("cudaMalloc (plan of several grids): ") + cudaGetErrorString(e);
+    return NSF_ERR_CUDA;
+  }
+  allocs.push_back(q);
   *p = static_cast<T*>(q);
   return NSF_OK;
 }
@@ -91,6 +86,145 @@ double lpt(std::vector<StageItem> items, int ctas, std::vector<StageItem>& order
   }
   return *std::max_element(load.begin(), load.end());
 }
+
+}  // namespace
+
+// A launch plan over several grids (an ensemble's members, an x-slab group's slabs): one stage launch over the
+// union of their work items, one fused boundary launch. members: handles whose device set-up is done with the
+// tile shape `tile`; the device allocations go to `allocs`; hGrids / *dGrids: the members' grids with the plan's
+// own norm slots.
+nsf_status build_members_plan(const std::vector<nsf_solver*>& members, int nSM, int tile, std::vector<void*>& allocs,
+                              LaunchPlan& L, std::vector<Grid>& hGrids, Grid** dGrids, std::string& err) {
+#define CKP(call)                                                    \
+  do {                                                               \
+    cudaError_t e_ = (call);                                         \
+    if (e_ != cudaSuccess) {                                         \
+      err = std::string(#call) + ": " + cudaGetErrorString(e_);      \
+      return NSF_ERR_CUDA;                                           \
+    }                                                                \
+  } while (0)
+  const int M = int(members.size());
+  L = LaunchPlan{};
+  L.nSM = nSM;
+  L.tile = tile;
+  const int TJ = stage_tile_j(tile), TK = stage_tile_k(tile);
+  const int ctas = nSM * std::max(1, stage_occupancy(tile));
+  // chunk length (planes per item, the same for every member): the one with the smallest LPT makespan
+  int maxPlanes = 1;
+  for (nsf_solver* s : members) maxPlanes = std::max(maxPlanes, int(s->setup.NI) - 2);
+  std::vector<StageItem> ordered;
+  std::vector<int> start;
+  double best = 1e300;
+  for (int len = maxPlanes; len >= std::min(4, maxPlanes); len = len > 16 ? len - 4 : len - 2) {
+    std::vector<StageItem> items;
+    for (int g = 0; g < M; ++g) member_items(members[g]->setup, g, TJ, TK, len, items);
+    std::vector<StageItem> o;
+    std::vector<int> st;
+    const double span = lpt(items, std::min(ctas, int(items.size())), o, st);
+    if (span < best - 1e-9) {
+      best = span;
+      ordered.swap(o);
+      start.swap(st);
+    }
+  }
+  L.stageSpan = int(best);
+  for (int g = 0; g < M; ++g)
+    mark_filter_planes(members[g]->hGrid, members[g]->filterNodes, TJ, TK, g, ordered);
+  L.nItems = int(ordered.size());
+  L.stageBlocks = int(start.size()) - 1;
+  nsf_status st;
+  if ((st = group_alloc(allocs, err, &L.items, ordered.size())) != NSF_OK) return st;
+  CKP(cudaMemcpy(L.items, ordered.data(), ordered.size() * sizeof(StageItem), cudaMemcpyHostToDevice));
+  if ((st = group_alloc(allocs, err, &L.ctaStart, start.size())) != NSF_OK) return st;
+  CKP(cudaMemcpy(L.ctaStart, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
+  // small kernels: block counts = maxima over the members
+  L.gfBlocks = std::max(8, 4 * nSM / M);  // grid-stride over each member's nodes
+  for (int a = 0; a < 3; ++a) {  // edge blocks: every member's own, member-major
+    std::vector<EdgeBlock> eb;
+    for (int g = 0; g < M; ++g) edge_blocks(members[g]->hGrid, members[g]->typeFlags.data(), g, a, eb);
+    L.nEdgeBlocks[a] = int(eb.size());
+    L.edgeBlocks[a] = nullptr;
+    if (eb.empty()) continue;
+    if ((st = group_alloc(allocs, err, &L.edgeBlocks[a], eb.size())) != NSF_OK) return st;
+    CKP(cudaMemcpy(L.edgeBlocks[a], eb.data(), eb.size() * sizeof(EdgeBlock), cudaMemcpyHostToDevice));
+  }
+  for (nsf_solver* s : members) {
+    const LaunchPlan& P = s->plan;
+    L.filterBlocks = std::max(L.filterBlocks, P.filterBlocks);
+    L.ghostBlocks = std::max(L.ghostBlocks, P.ghostBlocks);
+    L.solidBlocks = std::max(L.solidBlocks, P.solidBlocks);
+    L.hasFilter |= P.hasFilter;
+    L.hasGhostWork |= P.hasGhostWork;
+    L.hasSolid |= P.hasSolid;
+  }
+  {  // fused boundary kernel: bcBlocks blocks per member, all members' blocks resident at once
+    std::vector<const BcMemberLevels*> lv;
+    for (nsf_solver* s : members) lv.push_back(&s->bcLevels);
+    BcFlat fl;
+    bc_flatten(lv, fl);
+    const std::vector<int> ranges = bc_block_ranges(fl, bc_capacity(nSM));
+    L.bcBlocks = ranges.empty() ? 0 : ranges.back();
+    L.bcLevels = fl.levels;
+    if (L.bcBlocks == 0)
+      for (nsf_solver* s : members)
+        if (s->setup.bodiesInteract) {
+          err = "ensemble members with interacting immersed bodies need the fused boundary kernel, and the "
+                   "members do not fit one launch of it";
+          return NSF_ERR_GEOMETRY;
+        }
+    if (L.bcBlocks > 0) {
+      int widest = 1;  // the most blocks one member has: its norm slots
+      for (int g = 0; g < M; ++g) widest = std::max(widest, ranges[size_t(g) + 1] - ranges[size_t(g)]);
+      L.filterBlocks = std::max(L.filterBlocks, widest);
+      auto up = [&](auto** p, const auto& v) -> nsf_status {
+        nsf_status r = group_alloc(allocs, err, p, v.size());
+        if (r != NSF_OK) return r;
+        if (!v.empty() && cudaMemcpy(*p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice) != cudaSuccess) {
+          err = "could not upload the fused boundary kernel's plan";
+          return NSF_ERR_CUDA;
+        }
+        return NSF_OK;
+      };
+      if ((st = up(&L.bcBlockStart, ranges)) != NSF_OK) return st;
+      if ((st = up(&L.bcMemberLevels, fl.memberLevels)) != NSF_OK) return st;
+      if ((st = up(&L.bcEdges, fl.edges)) != NSF_OK) return st;
+      if ((st = up(&L.bcEdgeStart, fl.edgeStart)) != NSF_OK) return st;
+      if ((st = up(&L.bcItems, fl.items)) != NSF_OK) return st;
+      if ((st = up(&L.bcItemStart, fl.itemStart)) != NSF_OK) return st;
+      if ((st = group_alloc(allocs, err, &L.bcSync, 2 * size_t(M) + 1)) != NSF_OK) return st;
+      CKP(cudaMemset(L.bcSync, 0, (2 * size_t(M) + 1) * sizeof(unsigned long long)));
+    }
+  }
+  // member grids: the stage kernel adds its norm partials into slot 0 of each member, the near-body
+  // filter's blocks (or the fused boundary kernel's) use slots 1 .. filterBlocks
+  hGrids.resize(M);
+  for (int g = 0; g < M; ++g) {
+    Grid G = members[g]->hGrid;
+    const int slots = 1 + L.filterBlocks;
+    double* norm = nullptr;
+    if ((st = group_alloc(allocs, err, &norm, 5 * size_t(slots))) != NSF_OK) return st;
+    CKP(cudaMemset(norm, 0, 5 * size_t(slots) * sizeof(double)));
+    G.normPart = norm;
+    G.nNormSlots = slots;
+    G.normSlotFilter = 1;
+    hGrids[g] = G;
+  }
+  if ((st = group_alloc(allocs, err, dGrids, size_t(M))) != NSF_OK) return st;
+  CKP(cudaMemcpy(*dGrids, hGrids.data(), M * sizeof(Grid), cudaMemcpyHostToDevice));
+  return NSF_OK;
+#undef CKP
+}
+
+namespace {
+
+#define CKE(call)                                                          \
+  do {                                                                     \
+    cudaError_t e_ = (call);                                               \
+    if (e_ != cudaSuccess) {                                               \
+      e->err = std::string(#call) + ": " + cudaGetErrorString(e_);         \
+      return NSF_ERR_CUDA;                                                 \
+    }                                                                      \
+  } while (0)
 
 // ------------------------------------------------------------------------------------------- autotune
 std::string device_name(int device) {
@@ -227,118 +361,10 @@ nsf_status build_ensemble(nsf_ensemble* e, const char* cache) {
   }
   CKE(cudaSetDevice(e->device));
   CKE(cudaDeviceSynchronize());
-  LaunchPlan& L = e->plan;
-  L = LaunchPlan{};
-  L.nSM = e->nSM;
-  L.tile = e->tile;
-  const int TJ = stage_tile_j(e->tile), TK = stage_tile_k(e->tile);
-  const int ctas = e->nSM * std::max(1, stage_occupancy(e->tile));
-  // chunk length (planes per item, the same for every member): the one with the smallest LPT makespan
-  int maxPlanes = 1;
-  for (nsf_solver* s : e->members) maxPlanes = std::max(maxPlanes, int(s->setup.NI) - 2);
-  std::vector<StageItem> ordered;
-  std::vector<int> start;
-  double best = 1e300;
-  int bestLen = maxPlanes;
-  for (int len = maxPlanes; len >= 4; len = len > 16 ? len - 4 : len - 2) {
-    std::vector<StageItem> items;
-    for (int g = 0; g < M; ++g) member_items(e->members[g]->setup, g, TJ, TK, len, items);
-    std::vector<StageItem> o;
-    std::vector<int> st;
-    const double span = lpt(items, std::min(ctas, int(items.size())), o, st);
-    if (span < best - 1e-9) {
-      best = span;
-      bestLen = len;
-      ordered.swap(o);
-      start.swap(st);
-    }
-  }
-  (void)bestLen;
-  for (int g = 0; g < M; ++g)
-    mark_filter_planes(e->members[g]->hGrid, e->members[g]->filterNodes, TJ, TK, g, ordered);
-  L.nItems = int(ordered.size());
-  L.stageBlocks = int(start.size()) - 1;
-  nsf_status st;
-  if ((st = ens_alloc(e, &L.items, ordered.size())) != NSF_OK) return st;
-  CKE(cudaMemcpy(L.items, ordered.data(), ordered.size() * sizeof(StageItem), cudaMemcpyHostToDevice));
-  if ((st = ens_alloc(e, &L.ctaStart, start.size())) != NSF_OK) return st;
-  CKE(cudaMemcpy(L.ctaStart, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
-  // small kernels: block counts = maxima over the members
-  L.gfBlocks = std::max(8, 4 * e->nSM / M);  // grid-stride over each member's nodes
-  for (int a = 0; a < 3; ++a) {  // edge blocks: every member's own, member-major
-    std::vector<EdgeBlock> eb;
-    for (int g = 0; g < M; ++g) edge_blocks(e->members[g]->hGrid, e->members[g]->typeFlags.data(), g, a, eb);
-    L.nEdgeBlocks[a] = int(eb.size());
-    L.edgeBlocks[a] = nullptr;
-    if (eb.empty()) continue;
-    if ((st = ens_alloc(e, &L.edgeBlocks[a], eb.size())) != NSF_OK) return st;
-    CKE(cudaMemcpy(L.edgeBlocks[a], eb.data(), eb.size() * sizeof(EdgeBlock), cudaMemcpyHostToDevice));
-  }
-  for (nsf_solver* s : e->members) {
-    const LaunchPlan& P = s->plan;
-    L.filterBlocks = std::max(L.filterBlocks, P.filterBlocks);
-    L.ghostBlocks = std::max(L.ghostBlocks, P.ghostBlocks);
-    L.solidBlocks = std::max(L.solidBlocks, P.solidBlocks);
-    L.hasFilter |= P.hasFilter;
-    L.hasGhostWork |= P.hasGhostWork;
-    L.hasSolid |= P.hasSolid;
-  }
-  {  // fused boundary kernel: bcBlocks blocks per member, all members' blocks resident at once
-    std::vector<const BcMemberLevels*> lv;
-    for (nsf_solver* s : e->members) lv.push_back(&s->bcLevels);
-    BcFlat fl;
-    bc_flatten(lv, fl);
-    const std::vector<int> ranges = bc_block_ranges(fl, bc_capacity(e->nSM));
-    L.bcBlocks = ranges.empty() ? 0 : ranges.back();
-    L.bcLevels = fl.levels;
-    if (L.bcBlocks == 0)
-      for (nsf_solver* s : e->members)
-        if (s->setup.bodiesInteract) {
-          e->err = "ensemble members with interacting immersed bodies need the fused boundary kernel, and the "
-                   "members do not fit one launch of it";
-          return NSF_ERR_GEOMETRY;
-        }
-    if (L.bcBlocks > 0) {
-      int widest = 1;  // the most blocks one member has: its norm slots
-      for (int g = 0; g < M; ++g) widest = std::max(widest, ranges[size_t(g) + 1] - ranges[size_t(g)]);
-      L.filterBlocks = std::max(L.filterBlocks, widest);
-      auto up = [&](auto** p, const auto& v) -> nsf_status {
-        nsf_status r = ens_alloc(e, p, v.size());
-        if (r != NSF_OK) return r;
-        if (!v.empty() && cudaMemcpy(*p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice) != cudaSuccess) {
-          e->err = "could not upload the fused boundary kernel's plan";
-          return NSF_ERR_CUDA;
-        }
-        return NSF_OK;
-      };
-      if ((st = up(&L.bcBlockStart, ranges)) != NSF_OK) return st;
-      if ((st = up(&L.bcMemberLevels, fl.memberLevels)) != NSF_OK) return st;
-      if ((st = up(&L.bcEdges, fl.edges)) != NSF_OK) return st;
-      if ((st = up(&L.bcEdgeStart, fl.edgeStart)) != NSF_OK) return st;
-      if ((st = up(&L.bcItems, fl.items)) != NSF_OK) return st;
-      if ((st = up(&L.bcItemStart, fl.itemStart)) != NSF_OK) return st;
-      if ((st = ens_alloc(e, &L.bcSync, 2 * size_t(M) + 1)) != NSF_OK) return st;
-      CKE(cudaMemset(L.bcSync, 0, (2 * size_t(M) + 1) * sizeof(unsigned long long)));
-    }
-  }
-  // member grids: the stage kernel adds its norm partials into slot 0 of each member, the near-body
-  // filter's blocks (or the fused boundary kernel's) use slots 1 .. filterBlocks
-  e->hGrids.resize(M);
-  for (int g = 0; g < M; ++g) {
-    Grid G = e->members[g]->hGrid;
-    const int slots = 1 + L.filterBlocks;
-    double* norm = nullptr;
-    if ((st = ens_alloc(e, &norm, 5 * size_t(slots))) != NSF_OK) return st;
-    CKE(cudaMemset(norm, 0, 5 * size_t(slots) * sizeof(double)));
-    G.normPart = norm;
-    G.nNormSlots = slots;
-    G.normSlotFilter = 1;
-    e->hGrids[g] = G;
-  }
-  if ((st = ens_alloc(e, &e->dGrids, size_t(M))) != NSF_OK) return st;
-  CKE(cudaMemcpy(e->dGrids, e->hGrids.data(), M * sizeof(Grid), cudaMemcpyHostToDevice));
+  nsf_status st = build_members_plan(e->members, e->nSM, e->tile, e->allocs, e->plan, e->hGrids, &e->dGrids, e->err);
+  if (st != NSF_OK) return st;
   CKE(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-  e->launchesPerStep = enqueue_ensemble_step(e->dGrids, M, L, e->stream, nullptr);
+  e->launchesPerStep = enqueue_ensemble_step(e->dGrids, M, e->plan, e->stream, nullptr);
   CKE(cudaStreamEndCapture(e->stream, &e->graph));
   CKE(cudaGraphInstantiate(&e->graphExec, e->graph, 0));
   return NSF_OK;

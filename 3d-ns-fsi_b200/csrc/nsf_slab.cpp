@@ -17,10 +17,12 @@
 //
 // A group lives in one process or spans several (one GPU each, nsf_slab_group_create_ranks): rank r holds
 // the consecutive slabs p with p * world / P == r. Each process's slabs share one device and one stream,
-// and a step is one CUDA graph; a transfer packs the plane into a staging buffer and unpacks it on the
-// receiving side (the buffers each step's roles select are read on the device) -- within a process the
-// two sides share the buffer, across processes NCCL send/recv moves it (captured in the graph, between
-// the pack and the unpack launches). The global reductions gather every slab's partials (NCCL all-gather
+// and a step is one CUDA graph that treats them as an ensemble's members: one stage launch over the union of their
+// work items (or one per slab, kSharedStageCost) and one boundary launch (Taylor-Green 96^3 in two slabs: 41 launches
+// and 410 us per step before, 303 us now; 64^3 in three 339, 162). A
+// transfer within the process copies the plane from slab to slab (the buffers each step's roles select are read on
+// the device); across processes it is packed into a staging buffer, moved by NCCL send/recv (captured in the graph)
+// and unpacked on the receiving side. The global reductions gather every slab's partials (NCCL all-gather
 // across processes) and combine them in slab order, so every process computes the same dt and norms.
 // The node values and the dt sequence equal the single-grid solve's bit for bit:
 // every node's dt terms are formed by the same kernel as in the whole grid (the periodic x faces' by their
@@ -54,7 +56,10 @@ struct nsf_slab_group {
   std::vector<int> lo, hi;         // the global planes slab p owns: its interior planes, plus the x faces at the ends
   std::vector<int> base;           // global plane of slab p's local plane 0 (= a[p] - 1)
   bool xPeriodic = false;
-  Grid* dGrids = nullptr;          // copies of this process's slabs' grids, device
+  LaunchPlan plan{};               // one stage and one boundary launch over this process's slabs
+  bool oneStage = true;            // false: a stage launch per slab (see kSharedStageCost)
+  std::vector<Grid> hGrids;        // this process's slabs' grids with the plan's norm slots
+  Grid* dGrids = nullptr;          // the same on the device
   double* dPart = nullptr;         // [9 x local slabs] this process's slab partials
   double* dGather = nullptr;       // [9 x maxLocal x world] every process's partials (several processes)
   int* dAt = nullptr;              // [P] where slab p's partials are (in dPart, or in dGather)
@@ -64,6 +69,8 @@ struct nsf_slab_group {
   std::vector<SlabTask> packStage, unpackStage, packWrap, unpackWrap, packFilter, unpackFilter;
   SlabTask* dTasks = nullptr;      // all task lists, device, in the order above
   size_t offs[7] = {0, 0, 0, 0, 0, 0, 0};
+  std::vector<SlabMove> direct[3];  // transfers within this process, per list
+  SlabMove* dDirect[3] = {nullptr, nullptr, nullptr};
   // NCCL moves of each list (0 halos, 1 periodic x faces, 2 filtered density), in the group's global order
   struct Move {
     bool send;   // send (else receive)
@@ -82,6 +89,13 @@ struct nsf_slab_group {
 };
 
 namespace {
+
+// One stage launch over all of a process's slabs, or one per slab: the planes the busiest block streams decide
+// (LaunchPlan::stageSpan). A launch over several grids takes about 14 % longer per plane (per-item coefficients in
+// shared memory); a launch of its own costs a slab about 2.5 planes of ring fill and drain. Measured, us per step of
+// Taylor-Green in slabs, per slab / all at once: 64^3 in 3 -- / 162, 96^3 in 2 303 / 304, 128^3 in 2 546 / 555, 160^3
+// in 4 995 / 935, 160^3 in 2 884 / 947, 256^3 in 2 2848 / 3258, 256^3 in 4 3007 / 3296.
+constexpr double kSharedStageCost = 1.14, kStageLaunchPlanes = 2.5;
 
 nsf_status gfail(nsf_slab_group* g, nsf_status st, const std::string& m) {
   g->err = m;
@@ -257,11 +271,17 @@ nsf_status build_group(nsf_slab_group* g, int P, const void* ncclId) {
     s->slabCons.clear();
     s->slabPrim.clear();
   }
-  // device copies of the slabs' grids (the reductions read them)
-  std::vector<Grid> hg;
-  for (nsf_solver* s : g->slabs) hg.push_back(s->hGrid);
-  if ((st = galloc(g, &g->dGrids, hg.size())) != NSF_OK) return st;
-  CKG(cudaMemcpy(g->dGrids, hg.data(), hg.size() * sizeof(Grid), cudaMemcpyHostToDevice));
+  if ((st = build_members_plan(g->slabs, g->slabs[0]->nSM, g->slabs[0]->plan.tile, g->allocs, g->plan, g->hGrids,
+                               &g->dGrids, g->err)) != NSF_OK)
+    return st;
+  double apart = 0;
+  for (nsf_solver* s : g->slabs) apart += s->plan.stageSpan + kStageLaunchPlanes;
+  g->oneStage = kSharedStageCost * g->plan.stageSpan < apart;
+  if (!g->oneStage) {  // each slab's own stage launches write its own norm slots
+    for (size_t l = 0; l < g->slabs.size(); ++l) g->hGrids[l] = g->slabs[l]->hGrid;
+    CKG(cudaMemcpy(g->dGrids, g->hGrids.data(), g->hGrids.size() * sizeof(Grid), cudaMemcpyHostToDevice));
+  }
+  if (g->plan.bcBlocks <= 0) return gfail(g, NSF_ERR_CUDA, "the slabs do not fit one launch of the boundary kernel");
   if ((st = galloc(g, &g->dRed, 9)) != NSF_OK) return st;
   if ((st = galloc(g, &g->dPart, size_t(9) * size_t(g->maxLocal))) != NSF_OK) return st;
   CKG(cudaMemset(g->dPart, 0, size_t(9) * size_t(g->maxLocal) * sizeof(double)));
@@ -289,10 +309,7 @@ nsf_status build_group(nsf_slab_group* g, int P, const void* ncclId) {
     const size_t words = size_t(x.which == SLAB_STAGE ? 5 : 1) * size_t(g->planeWords);
     const bool fromHere = local(x.from), toHere = local(x.to);
     if (fromHere && toHere && !g->ncclAll) {
-      double* buf = nullptr;
-      if ((st = galloc(g, &buf, words)) != NSF_OK) return st;
-      pk.push_back(SlabTask{gridOf(x.from), x.fromPlane, x.which, buf});
-      up.push_back(SlabTask{gridOf(x.to), x.toPlane, x.which, buf});
+      g->direct[x.list].push_back(SlabMove{gridOf(x.from), gridOf(x.to), x.fromPlane, x.toPlane, x.which});
       continue;
     }
     if (fromHere) {
@@ -326,6 +343,11 @@ nsf_status build_group(nsf_slab_group* g, int P, const void* ncclId) {
   g->offs[6] = all.size();
   if ((st = galloc(g, &g->dTasks, all.size())) != NSF_OK) return st;
   CKG(cudaMemcpy(g->dTasks, all.data(), all.size() * sizeof(SlabTask), cudaMemcpyHostToDevice));
+  for (int q = 0; q < 3; ++q) {
+    if (g->direct[q].empty()) continue;
+    if ((st = galloc(g, &g->dDirect[q], g->direct[q].size())) != NSF_OK) return st;
+    CKG(cudaMemcpy(g->dDirect[q], g->direct[q].data(), g->direct[q].size() * sizeof(SlabMove), cudaMemcpyHostToDevice));
+  }
   CKG(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   CKG(cudaDeviceSynchronize());
   // one step as a CUDA graph
@@ -351,30 +373,40 @@ nsf_status build_group(nsf_slab_group* g, int P, const void* ncclId) {
     const ncclResult_t e = nccl->groupEnd();
     if (nr == ncclSuccess) nr = e;
   };
-  for (nsf_solver* s : g->slabs) launches += enqueue_step_begin(s->dGrid, s->plan, g->stream);
-  copies(4, 0, 0);  // filtered density halos (filter steps)
-  move(2);
-  copies(5, 0, 1);
-  for (int q = 0; q < 4; ++q) {
-    for (nsf_solver* s : g->slabs) {
-      launch_stage(s->hGrid, s->plan, q, g->stream);
+  auto exchange = [&](int list, int s) {  // list 0 halos, 1 periodic x faces, 2 filtered density
+    if (!g->direct[list].empty()) {
+      launch_slab_move(g->dDirect[list], int(g->direct[list].size()), g->planeWords, s, g->stream);
       ++launches;
     }
-    copies(2, q, 0);  // periodic x faces
-    move(1);
-    copies(3, q, 1);
-    for (nsf_solver* s : g->slabs) launches += launch_bc_part(s->dGrid, s->plan, q, false, g->stream);
-    copies(0, q, 0);  // halos
-    move(0);
-    copies(1, q, 1);
+    copies(2 * list, s, 0);
+    move(list);
+    copies(2 * list + 1, s, 1);
+  };
+  launches += enqueue_step_begin(g->dGrids, nLocal, g->plan, g->stream);
+  exchange(2, 0);
+  for (int q = 0; q < 4; ++q) {
+    if (g->oneStage) {
+      launch_stage_ensemble(g->dGrids, g->plan, q, g->stream);
+      ++launches;
+    } else {
+      for (size_t l = 0; l < g->slabs.size(); ++l) {
+        launch_stage(g->hGrids[l], g->slabs[l]->plan, q, g->stream);
+        ++launches;
+      }
+    }
+    exchange(1, q);
+    launches += launch_bc_part(g->dGrids, nLocal, g->plan, q, false, g->stream);
+    exchange(0, q);
   }
-  launch_slab_partials(g->dGrids, nLocal, g->dPart, g->stream);
-  if (useNccl && nr == ncclSuccess)
-    nr = nccl->allGather(g->dPart, g->dGather, size_t(9) * g->maxLocal, ncclDouble, static_cast<ncclComm_t>(g->comm),
-                         g->stream);
-  launch_slab_combine(useNccl ? g->dGather : g->dPart, g->dAt, P, g->dRed, g->stream);
-  launch_slab_finalize(g->dGrids, nLocal, g->dRed, g->stream);
-  launches += 3;
+  if (useNccl) {
+    launch_slab_partials(g->dGrids, nLocal, g->dPart, g->stream);
+    ++launches;
+    if (nr == ncclSuccess)
+      nr = nccl->allGather(g->dPart, g->dGather, size_t(9) * g->maxLocal, ncclDouble, static_cast<ncclComm_t>(g->comm),
+                           g->stream);
+  }
+  launch_slab_end(g->dGrids, nLocal, useNccl ? g->dGather : g->dPart, g->dAt, P, g->dRed, !useNccl, g->stream);
+  ++launches;
   if (nr != ncclSuccess) {
     cudaGraph_t dropped = nullptr;
     cudaStreamEndCapture(g->stream, &dropped);
@@ -534,21 +566,13 @@ nsf_status nsf_slab_group_download(nsf_slab_group* g, uint32_t mask, double* hos
   if (!g || !host || g->slabs.empty()) return NSF_ERR_ARG;
   CKG(cudaSetDevice(g->device));
   CKG(cudaStreamSynchronize(g->stream));
+  // every slab's owned planes straight to their place in the caller's array
   const HostSetup& W = g->whole;
-  const size_t plane = W.NJ * W.NK;
-  int nf = 0;
-  for (int f = 0; f < NSF_NUM_FIELDS; ++f) nf += (mask >> f) & 1;
   for (size_t l = 0; l < g->slabs.size(); ++l) {
     const size_t p = size_t(g->first) + l;
-    nsf_solver* s = g->slabs[l];
-    std::vector<double> loc(size_t(nf) * s->setup.N);
-    const nsf_status st = nsf_download(s, mask, loc.data());
-    if (st != NSF_OK) return gfail(g, st, s->err);
-    const int b0 = g->base[p];
-    for (int q = 0; q < nf; ++q)
-      for (int i = g->lo[p]; i <= g->hi[p]; ++i)
-        std::memcpy(host + size_t(q) * W.N + size_t(i) * plane, loc.data() + size_t(q) * s->setup.N + size_t(i - b0) * plane,
-                    plane * sizeof(double));
+    const nsf_status st = nsf_download_planes(g->slabs[l], mask, size_t(g->lo[p] - g->base[p]),
+                                              size_t(g->hi[p] - g->lo[p] + 1), host + size_t(g->lo[p]) * W.NJ * W.NK, W.N);
+    if (st != NSF_OK) return gfail(g, st, g->slabs[l]->err);
   }
   return NSF_OK;
 }

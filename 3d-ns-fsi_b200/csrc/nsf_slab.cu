@@ -45,9 +45,35 @@ __global__ void k_slab_copy(const SlabTask* __restrict__ tasks, int s, int dir) 
   }
 }
 
+// Planes that stay within the process: source plane straight to destination plane, blockIdx.y = task. A list's
+// tasks write planes that none of them reads.
+__global__ void k_slab_move(const SlabMove* __restrict__ tasks, int s) {
+  const SlabMove t = tasks[blockIdx.y];
+  const StepCtl* a = t.from->ctl;
+  const StepCtl* b = t.to->ctl;
+  if (!a->active) return;
+  const long long plane = t.from->sI;
+  const long long from = t.fromPlane * plane, to = t.toPlane * plane;
+  if (t.which == SLAB_FILTER) {
+    if (!a->filterNow) return;
+    const double* src = a->gfDst + from;
+    double* dst = b->gfDst + to;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < plane; q += (long long)gridDim.x * blockDim.x)
+      dst[q] = src[q];
+    return;
+  }
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < plane; q += (long long)gridDim.x * blockDim.x) {
+    double v[5];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) v[f] = a->O[s][f][from + q];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) b->O[s][f][to + q] = v[f];
+  }
+}
+
 // Each slab of this process: part[9 g .. 9 g + 8] = its four dt maxima (c + |u|, c + |v|, c + |w|, the
 // viscous term) and its five change-norm sums (its partial slots in order). One block.
-__global__ void k_slab_partials(const Grid* __restrict__ grids, int n, double* __restrict__ part) {
+__device__ void slab_partials(const Grid* __restrict__ grids, int n, double* part) {
   __shared__ double red[5 * 32];
   __shared__ double tot[5];
   for (int g = 0; g < n; ++g) {
@@ -67,9 +93,7 @@ __global__ void k_slab_partials(const Grid* __restrict__ grids, int n, double* _
 // The step's global quantities from every slab's partials (slab p's at part[9 at[p]]): out[0..3] the
 // largest dt maxima, out[4..8] the change-norm sums, slabs in order -- the same arithmetic whichever
 // process holds which slab. One thread.
-__global__ void k_slab_combine(const double* __restrict__ part, const int* __restrict__ at, int P,
-                               double* __restrict__ out) {
-  if (threadIdx.x != 0) return;
+__device__ void slab_combine(const double* part, const int* __restrict__ at, int P, double* out) {
   double mx[4] = {0, 0, 0, 0};
   double sum[5] = {0, 0, 0, 0, 0};
   for (int p = 0; p < P; ++p) {
@@ -83,8 +107,7 @@ __global__ void k_slab_combine(const double* __restrict__ part, const int* __res
 
 // End of step for every slab from the global quantities (finalize_grid's arithmetic): next dt, t, level,
 // history row -- the same values in every slab's control block.
-__global__ void k_slab_finalize(Grid* grids, int n, const double* __restrict__ in) {
-  if (threadIdx.x != 0) return;
+__device__ void slab_finalize(Grid* grids, int n, const double* in) {
   for (int g = 0; g < n; ++g) {
     Grid* gp = grids + g;
     StepCtl* c = gp->ctl;
@@ -108,7 +131,26 @@ __global__ void k_slab_finalize(Grid* grids, int n, const double* __restrict__ i
   }
 }
 
+__global__ void k_slab_partials(const Grid* __restrict__ grids, int n, double* __restrict__ part) {
+  slab_partials(grids, n, part);
+}
+
+// The end of a step: combine and finalize, by one thread. local: the partials are this process's own slabs' and
+// are formed first (one process; several gather them between the two launches).
+__global__ void k_slab_end(Grid* grids, int n, double* part, const int* __restrict__ at, int P, double* out, int local) {
+  if (local) slab_partials(grids, n, part);  // ends with a block barrier
+  if (threadIdx.x != 0) return;
+  slab_combine(part, at, P, out);
+  slab_finalize(grids, n, out);
+}
+
 }  // namespace
+
+void launch_slab_move(const SlabMove* tasks, int ntasks, long long planeWords, int s, void* stream) {
+  if (ntasks <= 0) return;
+  const long long b = (planeWords + 255) / 256;
+  k_slab_move<<<dim3(unsigned(b < 256 ? b : 256), unsigned(ntasks)), 256, 0, static_cast<cudaStream_t>(stream)>>>(tasks, s);
+}
 
 void launch_slab_copy(const SlabTask* tasks, int ntasks, long long planeWords, int s, int dir, void* stream) {
   if (ntasks <= 0) return;
@@ -121,12 +163,8 @@ void launch_slab_partials(const Grid* grids, int n, double* part, void* stream) 
   k_slab_partials<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(grids, n, part);
 }
 
-void launch_slab_combine(const double* part, const int* at, int P, double* out, void* stream) {
-  k_slab_combine<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(part, at, P, out);
-}
-
-void launch_slab_finalize(Grid* grids, int n, const double* in, void* stream) {
-  k_slab_finalize<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(grids, n, in);
+void launch_slab_end(Grid* grids, int n, double* part, const int* at, int P, double* out, bool local, void* stream) {
+  k_slab_end<<<1, local ? 256 : 32, 0, static_cast<cudaStream_t>(stream)>>>(grids, n, part, at, P, out, local ? 1 : 0);
 }
 
 }  // namespace nsf

@@ -19,16 +19,23 @@ struct SlabTask {
   double* buf;
 };
 
+// A plane transfer within the process, without a staging buffer.
+struct SlabMove {
+  const Grid* from;
+  const Grid* to;
+  int fromPlane, toPlane;
+  int which;
+};
+void launch_slab_move(const SlabMove* tasks, int ntasks, long long planeWords, int s, void* stream);
 // dir 0: pack the tasks' planes into their buffers; dir 1: unpack buffers into planes. planeWords: the
 // largest sI of the tasks' grids.
 void launch_slab_copy(const SlabTask* tasks, int ntasks, long long planeWords, int s, int dir, void* stream);
 // part[9 g ..]: grid g's four dt maxima and five change-norm sums.
 void launch_slab_partials(const Grid* grids, int n, double* part, void* stream);
-// out[0..3]: the dt maxima over all slabs, out[4..8]: the change-norm sums in slab order; slab p's partials
-// at part[9 at[p] ..].
-void launch_slab_combine(const double* part, const int* at, int P, double* out, void* stream);
-// The end of step of every grid from those global quantities.
-void launch_slab_finalize(Grid* grids, int n, const double* in, void* stream);
+// The end of step of n grids: out[0..3] the dt maxima over all P slabs, out[4..8] the change-norm sums in slab order
+// (slab p's partials at part[9 at[p] ..]), and the next dt, t, level and history row of every grid from them.
+// local: part holds this process's slabs' partials alone and is filled first.
+void launch_slab_end(Grid* grids, int n, double* part, const int* at, int P, double* out, bool local, void* stream);
 
 }  // namespace nsf
 #endif

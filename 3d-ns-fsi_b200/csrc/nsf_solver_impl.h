@@ -72,6 +72,12 @@ void nsf_adjoint_free(nsf_solver* s);
 // Device set-up of a handle whose host setup (s->setup) is in place (nsf_capi.cpp), and the initial dt of a
 // grid from its initial fields (Solver::updateTimeStepSize at t = 0).
 nsf_status nsf_build_device(nsf_solver* s);
+// The fields of `mask` at the handle's planes first .. first + count - 1 (reference layout) to host + q * pitch for
+// the q-th field (pitch in doubles); waits for the copies (nsf_capi.cpp).
+nsf_status nsf_download_planes(nsf_solver* s, uint32_t mask, size_t first, size_t count, double* host, size_t pitch);
+// One launch plan over several handles' grids (nsf_ensemble.cpp).
+nsf_status build_members_plan(const std::vector<nsf_solver*>& members, int nSM, int tile, std::vector<void*>& allocs,
+                              nsf::LaunchPlan& L, std::vector<nsf::Grid>& hGrids, nsf::Grid** dGrids, std::string& err);
 double nsf_initial_dt(const nsf_config& c, const nsf::HostSetup& S, const std::vector<double>& cons,
                       const std::vector<double>& prim);
 

@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(NT, 1) k_step(const __grid_constant__ Grid G0,
   __shared__ double tot[NQ];
   __shared__ __align__(16) unsigned char gsm[sizeof(Grid)];
   __shared__ __align__(16) unsigned char csm[sizeof(StepCtl)];
-  __shared__ StageItem tiles[kTileStash];
+  __shared__ __align__(16) unsigned char tsm[kTileStash * sizeof(StageItem)];
   __shared__ int levelCount[kStash];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   StepCtl* const gc = G0.ctl;
@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(NT, 1) k_step(const __grid_constant__ Grid G0,
   const Grid& G = *reinterpret_cast<const Grid*>(gsm);
   StepCtl& cs = *reinterpret_cast<StepCtl*>(csm);
   const int itBegin = P.start[blockIdx.x], nTiles = P.start[blockIdx.x + 1] - itBegin;
+  StageItem* const tiles = reinterpret_cast<StageItem*>(tsm);
   if (tid < kTileStash && tid < nTiles) tiles[tid] = P.items[itBegin + tid];
   auto tile = [&](int q) { return q < kTileStash ? tiles[q] : P.items[itBegin + q]; };
   // warps are numbered across the blocks, so that a short list of boundary items spreads over all SMs
