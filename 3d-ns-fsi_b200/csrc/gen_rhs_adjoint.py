@@ -12,6 +12,9 @@ with the reference's stencil coefficients. From it this script emits
   * numpy versions of the forward RHS and of the same gather (forward() and adjoint() below), used by
     the tests as an independent check of the emitted code and of the term table against the oracle.
 
+The adjoint kernel evaluates the same transposed stencil in flux form (nsf_rhs_adjoint_flux.cuh, about a quarter of the
+operations); the tests compare it with the numpy gather here.
+
     python 3d-ns-fsi_b200/csrc/gen_rhs_adjoint.py      (rewrites nsf_rhs_adjoint.cuh)
 """
 import itertools

@@ -191,7 +191,7 @@ nsf_status setup(nsf_solver* s) {
   if ((st = aalloc(s, a, &a->lamFnew, 2 * F)) != NSF_OK) return st;
   if ((st = aalloc(s, a, &a->lamInflow, plane)) != NSF_OK) return st;
   if ((st = aalloc(s, a, &a->tmpLam, 5 * N)) != NSF_OK) return st;
-  if ((st = aalloc(s, a, &a->tmpV, 11 * N)) != NSF_OK) return st;
+  if ((st = aalloc(s, a, &a->tmpV, 10 * N)) != NSF_OK) return st;
   if ((st = aalloc(s, a, &a->ipbar, 5 * NG)) != NSF_OK) return st;
   if ((st = aalloc(s, a, &a->fbar, 2 * plane)) != NSF_OK) return st;
   if ((st = aalloc(s, a, &a->bcSync, 2)) != NSF_OK) return st;

@@ -20,7 +20,7 @@
 #include "nsf_device.cuh"
 #include "nsf_internal.h"
 #include "nsf_physics.cuh"
-#include "nsf_rhs_adjoint.cuh"
+#include "nsf_rhs_adjoint_flux.cuh"
 
 namespace nsf {
 namespace {
@@ -228,16 +228,26 @@ __device__ __forceinline__ void adj_edge_item(const Grid& G, const EdgeBlock& eb
     // rho = f (filtered extrapolation); u_axis = ramp * M0 * profile; T = 0; p = rho / gamma
     for (int f = 0; f < 5; ++f) lam[f] = A.lamO[f][n];
     const long long s1 = ax1 == 0 ? G.sI : G.sJ, s2 = ax2 == 1 ? G.sJ : 1;
-    auto ext = [&](long long m) {
-      return 2 * val[0][side == 0 ? m + st : m - st] - val[0][side == 0 ? m + 2 * st : m - 2 * st];
-    };
+    // (a neighbour outside the box reads the node's own values, which are not used)
+    const bool has[4] = {a < b[2 * ax1 + 1], a > b[2 * ax1], bb < b[2 * ax2 + 1], bb > b[2 * ax2]};
+    const long long off[4] = {s1, -s1, s2, -s2};
+    double r1[5], r2[5];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const long long m = q < 4 && has[q & 3] ? n + off[q & 3] : n;
+      r1[q] = val[0][side == 0 ? m + st : m - st];
+      r2[q] = val[0][side == 0 ? m + 2 * st : m - 2 * st];
+    }
+    auto ext = [&](int q) { return 2 * r1[q] - r2[q]; };
     double f = 0;
     unsigned nn = 0;
-    if (a < b[2 * ax1 + 1]) { f += ext(n + s1); ++nn; }
-    if (a > b[2 * ax1]) { f += ext(n - s1); ++nn; }
-    if (bb < b[2 * ax2 + 1]) { f += ext(n + s2); ++nn; }
-    if (bb > b[2 * ax2]) { f += ext(n - s2); ++nn; }
-    f += nn * ext(n);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (has[q]) {
+        f += ext(q);
+        ++nn;
+      }
+    f += nn * ext(4);
     f /= 2 * nn;
     const double ramp = fmin(1., stageT / 10.) * C.m0 * (side == 1 ? -1.0 : 1.0);
     const double prof = (G.inflow && axis == 0) ? G.inflow[a * G.NKp + bb] : 1.0;
@@ -305,16 +315,18 @@ __device__ __forceinline__ void adj_prepare_item(const Grid& G, const AdjPtrs& A
   const double m1 = A.val[1][n], m2 = A.val[2][n], m3 = A.val[3][n], e4 = A.val[4][n];
   double rho = A.valR[n], rE = e4;
   double o[5], acc[5], u0[5], oz[5] = {0, 0, 0, 0, 0}, oy[5] = {0, 0, 0, 0, 0};
+  for (int f = 0; f < 5; ++f) {  // whatever the node's type, which is still on its way
+    o[f] = A.lamO[f][n];
+    acc[f] = A.lamAcc[f][n];
+    u0[f] = A.lamU0[f][n];
+  }
   // the z and y copies the stage kernel wrote with this node
   const bool zCopy = (ty & (ZCOPY_UP_BIT | ZCOPY_DOWN_BIT)) != 0;
   const long long nz = (ty & ZCOPY_UP_BIT) ? n + (G.NK - 2) : n - (G.NK - 2);
   const bool yCopy = (ty & YCOPY_BIT) != 0;
-  const long long ny = (n % G.sI) / G.sJ == 1 ? n + (G.NJ - 2) * G.sJ : n - (G.NJ - 2) * G.sJ;
+  const long long ny = yCopy && (n % G.sI) / G.sJ == 1 ? n + (G.NJ - 2) * G.sJ : n - (G.NJ - 2) * G.sJ;
   if (interior)
     for (int f = 0; f < 5; ++f) {
-      o[f] = A.lamO[f][n];
-      acc[f] = A.lamAcc[f][n];
-      u0[f] = A.lamU0[f][n];
       if (zCopy) oz[f] = A.lamO[f][nz];
       if (yCopy) oy[f] = A.lamO[f][ny];
     }
@@ -330,8 +342,8 @@ __device__ __forceinline__ void adj_prepare_item(const Grid& G, const AdjPtrs& A
     A.lamFnew[2 * f + 1] = 0.0;
   }
   const Prim pr = prims_of_nr(G.C, rho, m1, m2, m3, rE);  // as the stage kernel's staging warps
-  const double q[11] = {m1, m2, m3, e4, pr.u, pr.v, pr.w, pr.p, pr.T, pr.mu, pr.ka};
-  for (int v = 4; v < 11; ++v) V[v * G.N + n] = q[v];  // 0..3 are the stage input's own values (A.val)
+  const double q[10] = {m1, m2, m3, e4, pr.u, pr.v, pr.w, pr.p, pr.T, pr.mu};
+  for (int v = 4; v < 10; ++v) V[v * G.N + n] = q[v];  // 0..3 are the stage input's own values (A.val)
   if (!interior) {
     for (int f = 0; f < 5; ++f) lam[f * G.N + n] = 0.0;
     const uint8_t t = ty & TYPE_MASK;
@@ -415,18 +427,28 @@ __global__ void __launch_bounds__(kAdjBcThreads)
   }
   if (!edgeChain) return;
   const double stageT = P.roles->stageT[s];
-  for (int axis = 2; axis >= 0; --axis)  // z, y, then x
-    if (barrier(P.nEdge[axis]))
-      for (int v = gtid; v < 64 * P.nEdge[axis]; v += nthr) {
-        const int lane = v & 63;
-        adj_edge_item(G, P.edges[axis][v >> 6], lane & 31, lane >> 5, A, P.edgeVal, axis, stageT, P.fbar,
-                      P.lamInflow);
-      }
-  if (barrier(P.inletGather ? P.nEdge[0] : 0))
-    for (int v = gtid; v < 64 * P.nEdge[0]; v += nthr) {
-      const int lane = v & 63;
-      adj_inlet_gather_item(G, P.edges[0][v >> 6], lane & 31, lane >> 5, A, P.fbar);
+  // each thread's first edge block of the coming phase is read before the barrier in front of it
+  const int lane = gtid & 63, e0 = gtid >> 6;
+  EdgeBlock eb{};
+  auto first = [&](int axis) {
+    if (e0 < P.nEdge[axis]) eb = P.edges[axis][e0];
+  };
+  auto blocks = [&](int axis, auto item) {  // a thread's lane is the same in every block it takes (64 divides nthr)
+    for (int q = e0; q < P.nEdge[axis]; q += nthr >> 6) {
+      if (q != e0) eb = P.edges[axis][q];
+      item();
     }
+  };
+  first(2);
+  for (int axis = 2; axis >= 0; --axis) {  // z, y, then x
+    if (barrier(P.nEdge[axis]))
+      blocks(axis, [&] {
+        adj_edge_item(G, eb, lane & 31, lane >> 5, A, P.edgeVal, axis, stageT, P.fbar, P.lamInflow);
+      });
+    first(axis > 0 ? axis - 1 : 0);
+  }
+  if (barrier(P.inletGather ? P.nEdge[0] : 0))
+    blocks(0, [&] { adj_inlet_gather_item(G, eb, lane & 31, lane >> 5, A, P.fbar); });
 }
 
 // The RK4 combine's adjoint and the RHS inputs: one thread per node.
@@ -478,123 +500,122 @@ __global__ void k_tape_copy(const StepCtl* __restrict__ ctl, const __grid_consta
     dst[m] = src[m];
 }
 
-// Transposed RHS (generated gather) and the chain rule through the primitive / transport values.
-// A block takes an 8 (j) x 32 (k) tile of nodes through a chunk of i-planes. The generated gather reads
-// the RHS adjoints at the 19 RHS nodes around a node and u, v, w, T, mu, kappa at its 7-point stencil:
-// those 11 fields are staged per plane with a one-node halo in a 3-plane ring in shared memory (so every
-// read is a shared-memory load at a fixed offset), the other inputs (momenta, rho_E, p) are read at the
-// node itself from global memory. Planes and halo nodes outside the grid are staged as zeros.
-constexpr int RT_J = 8, RT_K = 32, RT_HK = RT_K + 2, RT_PLANE = (RT_J + 2) * RT_HK;
-constexpr int RT_FIELDS = 11;                     // RHS adjoints 0..4, then u, v, w, T, mu, kappa
-constexpr int RT_SLOT = RT_FIELDS * RT_PLANE;     // doubles per staged plane
-constexpr int RT_SMEM = 3 * RT_SLOT * 8;          // bytes: 89,760
-constexpr int kAdjRhsBlocks = 2;                  // resident blocks per SM (shared memory and registers)
-__host__ __device__ constexpr int rt_field(int q) {  // input quantity q -> staged field, or -1
-  return q == 4 ? 5 : q == 5 ? 6 : q == 6 ? 7 : q == 8 ? 8 : q == 9 ? 9 : q == 10 ? 10 : -1;
+// Transposed RHS (flux form, nsf_rhs_adjoint_flux.cuh) and the chain rule through the primitive / transport values.
+// A block takes 16 (k) x 4 (j) x 4 (i) nodes, one a thread: the RHS adjoints, u, v, w, T and mu of the nodes and a
+// one-node halo come into shared memory by asynchronous copies, all in one round trip. Three blocks an SM overlap one's
+// copies with another's arithmetic. The other inputs (momenta, rho_E, p) are read at the node itself. Halo nodes outside
+// the grid are staged as zeros.
+// What bounds it: L2 traffic (about 340 bytes a node, halos included) and the latency of the copies. Measured (64^3, 100
+// steps of the backward run from the tape, ms): 32.9 with the term-by-term gather over 19 RHS nodes marching along i,
+// 29.0 for the flux form marching along i with asynchronous plane copies, 26.9 with 16 x 8 x 4 nodes and two a thread
+// (two blocks of 112 registers), 25.8 now (80 registers).
+constexpr int RT_K = 16, RT_J = 4, RT_L = 4, RT_THREADS = RT_K * RT_J * RT_L;
+constexpr int RT_ROW = RT_K + 4;                      // a staged row: k0 - 1 at 1, k0 .. k0 + 15 at 2 (16-byte aligned) ..
+constexpr int RT_PLANE = (RT_J + 2) * RT_ROW;         // doubles per field and staged plane
+constexpr int RT_FIELDS = 10;                         // RHS adjoints 0..4, then u, v, w, T, mu
+constexpr int RT_SLOT = RT_FIELDS * RT_PLANE;
+constexpr int RT_SMEM = (RT_L + 2) * RT_SLOT * 8;     // bytes: 57,600
+constexpr int kAdjRhsBlocks = 3;                      // resident blocks per SM (registers and shared memory)
+
+// 8 or 16 bytes from global to shared memory, asynchronously; zeros if !in.
+__device__ __forceinline__ void copy8_async(double* dst, const double* src, bool in) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void copy16_async(double* dst, const double* src, int bytes) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
 
-__global__ void __launch_bounds__(32 * RT_J, kAdjRhsBlocks)
+__global__ void __launch_bounds__(RT_THREADS, kAdjRhsBlocks)
     k_adj_rhs(const Grid* __restrict__ gp, const __grid_constant__ Consts C, AdjPtrs A, const double* __restrict__ lam,
-              const double* __restrict__ V, int chunk) {
-  extern __shared__ double sm[];
+              const double* __restrict__ V) {
+  extern __shared__ __align__(16) double sm[];
   const Grid& G = *gp;
   const long long N = G.N, sI = G.sI, sJ = G.sJ;
   const int NI = G.NI, NJ = G.NJ, NK = G.NK;
   const int tilesK = (NK + RT_K - 1) / RT_K;
-  const int j0 = (blockIdx.x / tilesK) * RT_J, k0 = (blockIdx.x % tilesK) * RT_K;
-  const int i0 = blockIdx.y * chunk, i1 = min(NI - 1, i0 + chunk - 1);
-  if (i0 > i1) return;  // uniform over the block
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
-  const int j = j0 + ty, k = k0 + tx;
-  auto stage = [&](int p, int slot) {
-    double* s = sm + slot * RT_SLOT;
-    for (int idx = tid; idx < RT_PLANE; idx += 32 * RT_J) {
-      const int hj = idx / RT_HK, jj = j0 - 1 + hj, kk = k0 - 1 + (idx - hj * RT_HK);
-      const bool in = p >= 0 && p < NI && jj >= 0 && jj < NJ && kk >= 0 && kk < NK;
+  const int j0 = (blockIdx.x / tilesK) * RT_J, k0 = (blockIdx.x % tilesK) * RT_K, i0 = blockIdx.y * RT_L;
+  const int tid = threadIdx.x;
+  {  // ten copies a row and field: eight aligned pairs of the tile's own nodes, the halo node on either side
+    constexpr int OPS = RT_K / 2 + 2, ROWS = (RT_L + 2) * (RT_J + 2);
+    for (int idx = tid; idx < ROWS * OPS; idx += RT_THREADS) {
+      const int row = idx / OPS, op = idx - row * OPS, pl = row / (RT_J + 2), hj = row - pl * (RT_J + 2);
+      const int p = i0 - 1 + pl, jj = j0 - 1 + hj;
+      const bool rowIn = p >= 0 && p < NI && jj >= 0 && jj < NJ;
+      const int kk = op < RT_K / 2 ? k0 + 2 * op : op == RT_K / 2 ? k0 - 1 : k0 + RT_K;
+      const bool in = rowIn && kk >= 0 && kk < NK;
       const long long n = in ? p * sI + jj * sJ + kk : 0;
-      double v[RT_FIELDS];
+      double* d = sm + pl * RT_SLOT + hj * RT_ROW + (kk - k0) + 2;
+      const int bytes = !in ? 0 : kk + 1 < NK ? 16 : 8;  // of a pair
 #pragma unroll
-      for (int e = 0; e < 5; ++e) v[e] = in ? lam[e * N + n] : 0.0;
-      v[5] = in ? V[4 * N + n] : 0.0;
-      v[6] = in ? V[5 * N + n] : 0.0;
-      v[7] = in ? V[6 * N + n] : 0.0;
-      v[8] = in ? V[8 * N + n] : 0.0;
-      v[9] = in ? V[9 * N + n] : 0.0;
-      v[10] = in ? V[10 * N + n] : 0.0;
-#pragma unroll
-      for (int f = 0; f < RT_FIELDS; ++f) s[f * RT_PLANE + idx] = v[f];
-    }
-  };
-  stage(i0 - 1, 0);
-  stage(i0, 1);
-  int cur = 1;  // ring slot of plane i
-  for (int i = i0; i <= i1; ++i) {
-    const int nxt = cur == 2 ? 0 : cur + 1, prv = cur == 0 ? 2 : cur - 1;
-    stage(i + 1, nxt);
-    __syncthreads();
-    if (j < NJ && k < NK) {
-      const int sb[3] = {prv * RT_SLOT, cur * RT_SLOT, nxt * RT_SLOT};  // planes i-1, i, i+1
-      const int c = (ty + 1) * RT_HK + tx + 1;
-      const long long m = i * sI + j * sJ + k;
-      auto lamAt = [&](int e, int di, int dj, int dk) { return sm[sb[di + 1] + e * RT_PLANE + c + dj * RT_HK + dk]; };
-      // the inputs read at X only (momenta, rho_E, p) and the node's type: loaded before the gather, so
-      // their latency overlaps it
-      const double xv[5] = {A.val[1][m], A.val[2][m], A.val[3][m], A.val[4][m], V[7 * N + m]};
-      const uint8_t tym = G.type[m];
-      const bool filt = (tym & FILTER_BIT) != 0;
-      const int fi = filt ? G.fidx[m] : 0;
-      const double rho = filt ? A.valFpre[2 * fi] : A.valR[m];
-      // the adjoints this node adds into (only this thread writes them in this kernel)
-      double* const dR = filt ? A.lamFpre + 2 * fi : A.lamR + m;      // density's
-      double* const dE = filt ? A.lamFpre + 2 * fi + 1 : nullptr;     // rho_E's, filter nodes
-      const double aI1 = A.lamI[1][m], aI2 = A.lamI[2][m], aI3 = A.lamI[3][m], aI4 = A.lamI[4][m];
-      const double aR = *dR, aE = filt ? *dE : 0.0;
-      auto valAt = [&](int q, int di, int dj, int dk) {
-        const int f = rt_field(q);
-        return f >= 0 ? sm[sb[di + 1] + f * RT_PLANE + c + dj * RT_HK + dk] : xv[q == 7 ? 4 : q];
-      };
-      // the per-RHS-node conditions also bound the compiler's scheduling regions (without them it
-      // interleaves all 19 blocks and runs out of registers)
-      auto inner = [&](int di, int dj, int dk) {
-        const int a = i - di, b = j - dj, d = k - dk;
-        return a >= 1 && a <= NI - 2 && b >= 1 && b <= NJ - 2 && d >= 1 && d <= NK - 2;
-      };
-      double bar[11];
-      rhs_adjoint_gather(C, lamAt, valAt, inner, bar);
-      // chain rule: u = m r1, p = gm1 (rE - (rho+1) K), T = (gamma p - rho) r1, mu = x sqrt(x) sc1/(re (T+sc1)),
-      // kappa = mu pf, with r1 = 1/(rho+1), K = |u|^2/2, x = 1 + T
-      // the density of the primitives: the stage's density input, or the pre-filter copy at filter nodes
-      const double r1 = recip_nr(rho + 1.0);
-      const int cc = sb[1] + c;  // this node in the staged plane
-      const double u = sm[cc + 5 * RT_PLANE], v = sm[cc + 6 * RT_PLANE], w = sm[cc + 7 * RT_PLANE],
-                   T = sm[cc + 8 * RT_PLANE];
-      const double K = 0.5 * (u * u + v * v + w * w);
-      double ub = bar[4], vb = bar[5], wb = bar[6], pb = bar[7], Tb = bar[8], mub = bar[9];
-      mub += C.pf * bar[10];
-      const double x = 1.0 + T, sx = sqrt_nr(x), den = T + C.sc1;
-      Tb += mub * C.sc1 * (1.5 * sx * den - x * sx) * recip_nr(C.re * den * den);
-      pb += C.gamma * r1 * Tb;
-      double rhob = -r1 * Tb - T * r1 * Tb;
-      double rEb = C.gm1 * pb;
-      rhob += -C.gm1 * K * pb;
-      const double Kb = -C.gm1 * (rho + 1.0) * pb;
-      ub += Kb * u;
-      vb += Kb * v;
-      wb += Kb * w;
-      rhob += -(u * ub + v * vb + w * wb) * r1;
-      A.lamI[1][m] = aI1 + (bar[0] + r1 * ub);
-      A.lamI[2][m] = aI2 + (bar[1] + r1 * vb);
-      A.lamI[3][m] = aI3 + (bar[2] + r1 * wb);
-      *dR = aR + rhob;
-      if (filt) {
-        A.lamI[4][m] = aI4 + bar[3];
-        *dE = aE + rEb;
-      } else {
-        A.lamI[4][m] = (aI4 + bar[3]) + rEb;
+      for (int f = 0; f < RT_FIELDS; ++f) {
+        // staged fields u, v, w, T, mu are rows 4, 5, 6, 8, 9 of V
+        const double* src = (f < 5 ? lam + f * N : V + (f < 8 ? f - 1 : f) * N) + n;
+        if (op < RT_K / 2)
+          copy16_async(d + f * RT_PLANE, src, bytes);
+        else
+          copy8_async(d + f * RT_PLANE, src, in);
       }
     }
-    __syncthreads();  // the next iteration restages the oldest slot
-    cur = nxt;
+  }
+  const int tx = tid % RT_K, ty = tid / RT_K % RT_J, grp = tid / (RT_K * RT_J);
+  const int j = j0 + ty, k = k0 + tx;
+  const int c = (ty + 1) * RT_ROW + tx + 2;
+  const int i = i0 + grp;
+  const bool mine = i < NI && j < NJ && k < NK;
+  const long long m = mine ? i * sI + j * sJ + k : 0;
+  // the node's filter slot (-1: not filtered), two dependent loads, while the copies travel
+  const int fi = mine && G.nFilter > 0 && (G.type[m] & FILTER_BIT) ? G.fidx[m] : -1;
+  const bool filt = fi >= 0;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  if (!mine) return;
+  const double mom[3] = {A.val[1][m], A.val[2][m], A.val[3][m]}, rE = A.val[4][m], p = V[7 * N + m];
+  const double rho = filt ? A.valFpre[2 * fi] : A.valR[m];
+  const double* const sC = sm + (grp + 1) * RT_SLOT + c;
+  auto lamAt = [&](int e, int di, int dj, int dk) { return sC[di * RT_SLOT + e * RT_PLANE + dj * RT_ROW + dk]; };
+  auto valAt = [&](int v, int di, int dj, int dk) { return sC[di * RT_SLOT + (5 + v) * RT_PLANE + dj * RT_ROW + dk]; };
+  auto inner = [&](int d, int o) {
+    return d == 0 ? i + o >= 1 && i + o <= NI - 2 : d == 1 ? j + o >= 1 && j + o <= NJ - 2 : k + o >= 1 && k + o <= NK - 2;
+  };
+  auto node = [&](int d) { return inner((d + 1) % 3, 0) && inner((d + 2) % 3, 0); };
+  auto face = [&](int d, int o) {
+    const int x = d == 0 ? i : d == 1 ? j : k, n = d == 0 ? NI : d == 1 ? NJ : NK;
+    return node(d) && x + o >= 0 && x + o < n;
+  };
+  const adj::Bar bar = adj::rhs_adjoint(C, lamAt, valAt, mom, rE, p, node, inner, face);
+  // the adjoints this node adds into (only this thread writes them in this kernel), on their way during the chain rule
+  double* const dR = filt ? A.lamFpre + 2 * fi : A.lamR + m;                // density's
+  double* const dE = filt ? A.lamFpre + 2 * fi + 1 : A.lamI[4] + m;         // that of rho_E in the primitives
+  const double aI1 = A.lamI[1][m], aI2 = A.lamI[2][m], aI3 = A.lamI[3][m], aI4 = A.lamI[4][m], aR = *dR, aE = *dE;
+  // chain rule: u = m r1, p = gm1 (rE - (rho+1) K), T = (gamma p - rho) r1, mu = x sqrt(x) sc1/(re (T+sc1)),
+  // with r1 = 1/(rho+1), K = |u|^2/2, x = 1 + T
+  // the density of the primitives: the stage's density input, or the pre-filter copy at filter nodes
+  const double r1 = recip_nr(rho + 1.0);
+  const double u = sC[5 * RT_PLANE], v = sC[6 * RT_PLANE], w = sC[7 * RT_PLANE], T = sC[8 * RT_PLANE];
+  const double K = 0.5 * (u * u + v * v + w * w);
+  double ub = bar.u[0], vb = bar.u[1], wb = bar.u[2], pb = bar.p, Tb = bar.T;
+  const double x = 1.0 + T, sx = sqrt_nr(x), den = T + C.sc1;
+  Tb += bar.mu * C.sc1 * (1.5 * sx * den - x * sx) * recip_nr(C.re * den * den);
+  pb += C.gamma * r1 * Tb;
+  double rhob = -r1 * Tb - T * r1 * Tb;
+  const double rEb = C.gm1 * pb;
+  rhob += -C.gm1 * K * pb;
+  const double Kb = -C.gm1 * (rho + 1.0) * pb;
+  ub += Kb * u;
+  vb += Kb * v;
+  wb += Kb * w;
+  rhob += -(u * ub + v * vb + w * wb) * r1;
+  A.lamI[1][m] = aI1 + (bar.m[0] + r1 * ub);
+  A.lamI[2][m] = aI2 + (bar.m[1] + r1 * vb);
+  A.lamI[3][m] = aI3 + (bar.m[2] + r1 * wb);
+  *dR = aR + rhob;
+  if (filt) {
+    A.lamI[4][m] = aI4 + bar.rE;
+    *dE = aE + rEb;
+  } else {
+    A.lamI[4][m] = (aI4 + bar.rE) + rEb;
   }
 }
 
@@ -711,15 +732,9 @@ int adj_kernels_init() {
 
 void launch_adj_rhs(const Grid* dg, const Grid& hg, const AdjPtrs& A, const double* lam, const double* V, int nSM,
                     void* stream) {
-  // i-chunks: enough blocks for kAdjRhsBlocks per SM, each chunk at least 4 planes (a chunk of L planes
-  // stages L + 2)
   const int tiles = ((hg.NJ + RT_J - 1) / RT_J) * ((hg.NK + RT_K - 1) / RT_K);
-  int chunks = (kAdjRhsBlocks * nSM + tiles - 1) / tiles;
-  chunks = std::max(1, std::min(chunks, hg.NI / 4));
-  const int chunk = (hg.NI + chunks - 1) / chunks;
-  chunks = (hg.NI + chunk - 1) / chunk;
-  k_adj_rhs<<<dim3(tiles, chunks), dim3(32, RT_J), RT_SMEM, static_cast<cudaStream_t>(stream)>>>(dg, hg.C, A, lam, V,
-                                                                                                   chunk);
+  k_adj_rhs<<<dim3(tiles, (hg.NI + RT_L - 1) / RT_L), RT_THREADS, RT_SMEM, static_cast<cudaStream_t>(stream)>>>(
+      dg, hg.C, A, lam, V);
 }
 
 void launch_copies(const double* const* src, double* const* dst, const long long* words, int count, int nSM,
