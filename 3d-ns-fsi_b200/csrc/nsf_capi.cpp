@@ -705,19 +705,6 @@ nsf_status build_device(nsf_solver* s) {
   return NSF_OK;
 }
 
-// Queues nsteps steps on the handle's stream: the whole-step kernel where the grid has one (launches of at most
-// kStepsPerLaunch steps, so that other streams' work gets its turn), else one graph launch per step.
-constexpr uint64_t kStepsPerLaunch = 64;
-nsf_status queue_steps(nsf_solver* s, uint64_t nsteps) {
-  if (s->plan.stepBlocks > 0) {
-    for (uint64_t q = 0; q < nsteps; q += kStepsPerLaunch)
-      CK(cudaError_t(launch_steps(s->hGrid, s->dGrid, s->plan, int(std::min(kStepsPerLaunch, nsteps - q)), s->stream)));
-    return NSF_OK;
-  }
-  for (uint64_t q = 0; q < nsteps; ++q) CK(cudaGraphLaunch(s->graphExec, s->stream));
-  return NSF_OK;
-}
-
 // Slots of the asked-for fields in a packed download (increasing field order), and how many there are.
 SnapSlots snap_slots(uint32_t mask, int* count) {
   SnapSlots sl;
@@ -733,6 +720,17 @@ SnapInactive snap_inactive(const nsf_solver* s) {
 
 
 }  // namespace
+
+nsf_status nsf_queue_steps(nsf_solver* s, uint64_t nsteps, const StepTape& tape) {
+  if (s->plan.stepBlocks > 0) {
+    constexpr uint64_t perLaunch = 64;  // so that other streams' work gets its turn
+    for (uint64_t q = 0; q < nsteps; q += perLaunch)
+      CK(cudaError_t(launch_steps(s->hGrid, s->dGrid, s->plan, int(std::min(perLaunch, nsteps - q)), s->stream, tape)));
+    return NSF_OK;
+  }
+  for (uint64_t q = 0; q < nsteps; ++q) CK(cudaGraphLaunch(s->graphExec, s->stream));
+  return NSF_OK;
+}
 
 // For the x-slab groups (nsf_slab.cpp): device set-up of a handle whose host setup is already in place,
 // and the initial dt of a whole grid.
@@ -856,7 +854,7 @@ nsf_status nsf_march(nsf_solver* s, uint64_t nsteps) {
     return NSF_ERR_STATE;
   }
   CK(cudaSetDevice(s->device));
-  return queue_steps(s, nsteps);
+  return nsf_queue_steps(s, nsteps);
 }
 
 nsf_status nsf_sync(nsf_solver* s) {
@@ -1103,7 +1101,7 @@ nsf_status nsf_march_timed(nsf_solver* s, uint64_t nsteps, double* elapsed_ms) {
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
   CK(cudaEventRecord(a, s->stream));
-  const nsf_status st = queue_steps(s, nsteps);
+  const nsf_status st = nsf_queue_steps(s, nsteps);
   if (st != NSF_OK) return st;
   CK(cudaEventRecord(b, s->stream));
   CK(cudaEventSynchronize(b));

@@ -260,7 +260,17 @@ size_t step_smem_bytes(int shape, int planes, int levels);
 StepChoice step_choose(int NI, int NJ, int NK, int nSM);
 int step_configure(int shape, size_t smem);
 int step_capacity(int shape, size_t smem, int nSM);
-int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream);
+// What the steps leave for the discrete adjoint (nsf_adjoint.cpp), or stage == NULL: per step one set of values, set
+// (time level mod nSets) at stage + set * setWords and result + set * setWords. A set holds, per stage s at s * perStage,
+// the stage input's five fields, the density of its primitives where that is another buffer, and (at 11 N) the near-body
+// filter's pre-filter values; result: the five fields the step ends with.
+struct StepTape {
+  double* stage = nullptr;
+  double* result = nullptr;
+  long long setWords = 0, perStage = 0;
+  int nSets = 1;
+};
+int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream, const StepTape& tape = {});
 
 // Host entry points of nsf_kernels.cu.
 // Stage-kernel variant queries (v: StageTile).

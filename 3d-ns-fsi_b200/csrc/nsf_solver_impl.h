@@ -72,6 +72,9 @@ void nsf_adjoint_free(nsf_solver* s);
 // Device set-up of a handle whose host setup (s->setup) is in place (nsf_capi.cpp), and the initial dt of a
 // grid from its initial fields (Solver::updateTimeStepSize at t = 0).
 nsf_status nsf_build_device(nsf_solver* s);
+// Queues nsteps steps on the handle's stream (nsf_capi.cpp): the whole-step kernel where the grid has one (with it, the
+// steps may leave their sets on a tape), else one graph launch per step.
+nsf_status nsf_queue_steps(nsf_solver* s, uint64_t nsteps, const nsf::StepTape& tape = {});
 // The fields of `mask` at the handle's planes first .. first + count - 1 (reference layout) to host + q * pitch for
 // the q-th field (pitch in doubles); waits for the copies (nsf_capi.cpp).
 nsf_status nsf_download_planes(nsf_solver* s, uint32_t mask, size_t first, size_t count, double* host, size_t pitch);

@@ -55,6 +55,7 @@ struct StepParams {
   const int* start;
   double* part;                // [NQ][blocks] end-of-step partials
   int stashOffset;             // bytes from the start of the dynamic shared memory to the item stash
+  StepTape tape;
   unsigned long long* sync;    // the grid barrier's arrival counter (see grid_barrier, nsf_physics.cuh)
 };
 
@@ -259,7 +260,27 @@ struct StepBarrier {
   }
 };
 
-template <class T>
+// words doubles (a multiple of 2, 16-byte aligned) from src to dst by all blocks; src is read through L2. A call: inlined
+// at each of its uses it would cost the stage phases their registers.
+__device__ __noinline__ void tape_copy(const double* src, double* dst, long long words, int gtid, int nthr) {
+  const double2* a = reinterpret_cast<const double2*>(src);
+  double2* b = reinterpret_cast<double2*>(dst);
+  const long long n = words / 2;
+  constexpr int U = 4;
+  for (long long q = gtid; q < n; q += (long long)U * nthr) {
+    double2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (q + (long long)u * nthr < n) v[u] = __ldcg(a + q + (long long)u * nthr);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (q + (long long)u * nthr < n) __stcs(b + q + (long long)u * nthr, v[u]);
+  }
+}
+
+// TAPE: the steps also record their sets (StepParams::tape): a stage's input right before the stage, which no block
+// writes until the stage after it, and the step's result after the end-of-step barrier.
+template <class T, bool TAPE>
 __global__ void __launch_bounds__(NT, 1) k_step(const __grid_constant__ Grid G0, Grid* gp,
                                                 const __grid_constant__ StepParams P, int nsteps) {
   extern __shared__ __align__(16) double sm[];
@@ -323,15 +344,25 @@ __global__ void __launch_bounds__(NT, 1) k_step(const __grid_constant__ Grid G0,
       for (long long n = gtid; n < G.N; n += nthr) density_filter_node(G, &cs, n);
       barrier();
     }
+    double* const set = TAPE ? P.tape.stage + (long long)(cs.level % (unsigned)P.tape.nSets) * P.tape.setWords : nullptr;
+    double* const setEnd = TAPE ? P.tape.result + (long long)(cs.level % (unsigned)P.tape.nSets) * P.tape.setWords : nullptr;
+    auto record = [&](int s) {
+      double* const base = set + s * P.tape.perStage;
+      for (int f = 0; f < 5; ++f) tape_copy(cs.I[s][f], base + f * G.N, G.N, gtid, nthr);
+      if (cs.R[s] != cs.I[s][0]) tape_copy(cs.R[s], base + 5 * G.N, G.N, gtid, nthr);
+      if (G.nFilter > 0) tape_copy(G.fpre, base + 11 * G.N, 2ll * G.nFilter, gtid, nthr);
+    };
     DtAcc dta;
     double nsum[5] = {0, 0, 0, 0, 0};
     int bad = 0;
 #pragma unroll 1
     for (int s = 0; s < 3; ++s) {
+      if (TAPE) record(s);
       for (int q = 0; q < nTiles; ++q) stage_tile<T, false>(G0, cs, s, tile(q), sm, dta, nsum, bad);
       boundary(std::false_type{}, s, dta, nsum, bad);
       barrier();
     }
+    if (TAPE) record(3);
     for (int q = 0; q < nTiles; ++q) stage_tile<T, true>(G0, cs, 3, tile(q), sm, dta, nsum, bad);
     boundary(std::true_type{}, 3, dta, nsum, bad);
     // end of step: this block's partials, then every block combines all of them in the same order
@@ -364,6 +395,8 @@ __global__ void __launch_bounds__(NT, 1) k_step(const __grid_constant__ Grid G0,
     if (blockIdx.x == 0 && tid >= 32 && tid < 39) history_entry(G, level, tNew, dtUsed, tot + 4, tid - 32);
     if (tid < 4) cs.mx[tid] = static_cast<unsigned long long>(__double_as_longlong(tot[tid]));
     if (tid == 0) finish_step(G, &cs, tot);
+    if (TAPE)
+      for (int f = 0; f < 5; ++f) tape_copy(cs.O[3][f], setEnd + f * G.N, G.N, gtid, nthr);
     __syncthreads();
   }
   if (blockIdx.x == 0) {  // the control block as the next call reads it; the flags other blocks set stay as they are
@@ -380,9 +413,10 @@ template <class T>
 StepShape shape_of() {
   return StepShape{T::TK, T::TJ, T::LMAX, T::HP};
 }
-const void* kernel_of(int shape) {
-  if (shape == STEP_TILE_THIN) return reinterpret_cast<const void*>(&k_step<Thin>);
-  return reinterpret_cast<const void*>(&k_step<Cube>);
+const void* kernel_of(int shape, bool tape) {
+  if (shape == STEP_TILE_THIN)
+    return tape ? reinterpret_cast<const void*>(&k_step<Thin, true>) : reinterpret_cast<const void*>(&k_step<Thin, false>);
+  return tape ? reinterpret_cast<const void*>(&k_step<Cube, true>) : reinterpret_cast<const void*>(&k_step<Cube, false>);
 }
 
 }  // namespace
@@ -420,16 +454,21 @@ StepChoice step_choose(int NI, int NJ, int NK, int nSM) {
 }
 
 int step_configure(int shape, size_t smem) {
-  return int(cudaFuncSetAttribute(kernel_of(shape), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  cudaError_t e = cudaSuccess;
+  for (bool tape : {false, true})
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel_of(shape, tape), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  return int(e);
 }
 
 int step_capacity(int shape, size_t smem, int nSM) {
-  int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel_of(shape), NT, smem) != cudaSuccess) return 0;
-  return nb * nSM;
+  int nb = 0, nb2 = 0;  // both instantiations run the same plan
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel_of(shape, false), NT, smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, kernel_of(shape, true), NT, smem) != cudaSuccess) return 0;
+  return std::min(nb, nb2) * nSM;
 }
 
-int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream) {
+int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream, const StepTape& tape) {
   StepParams P{};
   P.bc.edges = L.bcEdges;
   P.bc.edgeStart = L.bcEdgeStart;
@@ -442,6 +481,7 @@ int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void
   P.part = L.stepPart;
   P.sync = L.stepSync;
   P.stashOffset = int(staged_bytes(L.stepShape, L.stepPlanes));
+  P.tape = tape;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(L.stepBlocks));
   cfg.blockDim = dim3(NT);
@@ -452,8 +492,9 @@ int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (L.stepShape == STEP_TILE_THIN) return int(cudaLaunchKernelEx(&cfg, k_step<Thin>, hg, dg, P, nsteps));
-  return int(cudaLaunchKernelEx(&cfg, k_step<Cube>, hg, dg, P, nsteps));
+  auto go = [&](auto kernel) { return int(cudaLaunchKernelEx(&cfg, kernel, hg, dg, P, nsteps)); };
+  if (L.stepShape == STEP_TILE_THIN) return tape.stage ? go(k_step<Thin, true>) : go(k_step<Thin, false>);
+  return tape.stage ? go(k_step<Cube, true>) : go(k_step<Cube, false>);
 }
 
 }  // namespace nsf
