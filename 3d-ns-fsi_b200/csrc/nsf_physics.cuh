@@ -278,31 +278,57 @@ __device__ __forceinline__ void x_face(const Consts& C, const XOwn& a, const XOw
   f[4] = __fma_rn(C.e_xx12, __dmul_rn(C.pf, __dmul_rn(ms, __dsub_rn(b.T, a.T))), e4);
 }
 
-// y- and z-direction part of the right-hand side at P (the reference's terms not covered by G and F).
-// cP/pP: staged centre plane; pE/pW: staged neighbour planes (only their N/S/U/D velocity values are
-// read, for the mixed x-derivatives at the in-plane neighbours); own: P's own values. The staged planes
-// hold u, v, w, p, T, mu (fields 0..5); kappa = pf mu is formed here, as prims_of forms it.
+// The velocities at a node's in-plane neighbours (N, S: +j, -j; U, D: +k, -k) that the mixed x-differences read, in
+// registers (Cross) or read from the staged plane at each use (CrossMem: plane pointer p, node c).
+struct Cross {
+  double vn, vs, un, us, wu, wd, uu, ud;
+  __device__ __forceinline__ double vN() const { return vn; }
+  __device__ __forceinline__ double vS() const { return vs; }
+  __device__ __forceinline__ double uN() const { return un; }
+  __device__ __forceinline__ double uS() const { return us; }
+  __device__ __forceinline__ double wU() const { return wu; }
+  __device__ __forceinline__ double wD() const { return wd; }
+  __device__ __forceinline__ double uU() const { return uu; }
+  __device__ __forceinline__ double uD() const { return ud; }
+};
 template <int HK, int FS>
-__device__ __forceinline__ void yz_part(const Consts& C, const double* __restrict__ cP, const double* __restrict__ pW,
-                                        const double* __restrict__ pP, const double* __restrict__ pE, int c,
-                                        const XOwn& own, double out[5]) {
+struct CrossMem {
+  const double* p;
+  int c;
+  __device__ __forceinline__ double vN() const { return p[1 * FS + c + HK]; }
+  __device__ __forceinline__ double vS() const { return p[1 * FS + c - HK]; }
+  __device__ __forceinline__ double uN() const { return p[0 * FS + c + HK]; }
+  __device__ __forceinline__ double uS() const { return p[0 * FS + c - HK]; }
+  __device__ __forceinline__ double wU() const { return p[2 * FS + c + 1]; }
+  __device__ __forceinline__ double wD() const { return p[2 * FS + c - 1]; }
+  __device__ __forceinline__ double uU() const { return p[0 * FS + c + 1]; }
+  __device__ __forceinline__ double uD() const { return p[0 * FS + c - 1]; }
+  __device__ __forceinline__ Cross load() const { return Cross{vN(), vS(), uN(), uS(), wU(), wD(), uU(), uD()}; }
+};
+// y- and z-direction part of the right-hand side at P (the reference's terms not covered by G and F).
+// cP/pP: staged centre plane; xW, xP, xE: the in-plane neighbours' velocities on the planes at -x, P and +x (of the
+// neighbour planes only these are read, for the mixed x-derivatives); own: P's own values. The staged planes
+// hold u, v, w, p, T, mu (fields 0..5); kappa = pf mu is formed here, as prims_of forms it.
+template <int HK, int FS, class X>
+__device__ __forceinline__ void yz_part(const Consts& C, const double* __restrict__ cP, const double* __restrict__ pP,
+                                        const X& xW, const X& xP, const X& xE, int c, const XOwn& own, double out[5]) {
   enum { RU = 1, RV = 2, RW = 3, RE = 4 };
   enum { U = 0, V = 1, W = 2, P = 3, TT = 4, MU = 5 };
 #define F_(b, v, o) (b)[(v)*FS + c + (o)]
   constexpr int oN = HK, oS = -HK, oU = 1, oD = -1;
   const double muP = own.mu, uP = own.u, vP = own.v, wP = own.w, TP = own.T;
   const double muN = F_(pP, MU, oN), muS = F_(pP, MU, oS), muU = F_(pP, MU, oU), muD = F_(pP, MU, oD);
-  const double uN = F_(pP, U, oN), uS = F_(pP, U, oS), uU = F_(pP, U, oU), uD = F_(pP, U, oD);
-  const double vN = F_(pP, V, oN), vS = F_(pP, V, oS), vU = F_(pP, V, oU), vD = F_(pP, V, oD);
-  const double wN = F_(pP, W, oN), wS = F_(pP, W, oS), wU = F_(pP, W, oU), wD = F_(pP, W, oD);
+  const double uN = xP.uN(), uS = xP.uS(), uU = xP.uU(), uD = xP.uD();
+  const double vN = xP.vN(), vS = xP.vS(), vU = F_(pP, V, oU), vD = F_(pP, V, oD);
+  const double wN = F_(pP, W, oN), wS = F_(pP, W, oS), wU = xP.wU(), wD = xP.wD();
   const double pN = F_(pP, P, oN), pS = F_(pP, P, oS), pU = F_(pP, P, oU), pD = F_(pP, P, oD);
   // face viscosity sums (mu_N + mu_P) ... of the normal viscous and heat-flux terms
   const double msN = muN + muP, msS = muS + muP, msU = muU + muP, msD = muD + muP;
   // mixed-derivative products mu_X (difference across X), shared by momentum and energy
-  const double mNdxv = muN * (F_(pE, V, oN) - F_(pW, V, oN)), mSdxv = muS * (F_(pE, V, oS) - F_(pW, V, oS));
-  const double mNdxu = muN * (F_(pE, U, oN) - F_(pW, U, oN)), mSdxu = muS * (F_(pE, U, oS) - F_(pW, U, oS));
-  const double mUdxw = muU * (F_(pE, W, oU) - F_(pW, W, oU)), mDdxw = muD * (F_(pE, W, oD) - F_(pW, W, oD));
-  const double mUdxu = muU * (F_(pE, U, oU) - F_(pW, U, oU)), mDdxu = muD * (F_(pE, U, oD) - F_(pW, U, oD));
+  const double mNdxv = muN * (xE.vN() - xW.vN()), mSdxv = muS * (xE.vS() - xW.vS());
+  const double mNdxu = muN * (xE.uN() - xW.uN()), mSdxu = muS * (xE.uS() - xW.uS());
+  const double mUdxw = muU * (xE.wU() - xW.wU()), mDdxw = muD * (xE.wD() - xW.wD());
+  const double mUdxu = muU * (xE.uU() - xW.uU()), mDdxu = muD * (xE.uD() - xW.uD());
   const double wNU = F_(pP, W, oN + oU), wND = F_(pP, W, oN + oD), wSU = F_(pP, W, oS + oU), wSD = F_(pP, W, oS + oD);
   const double vNU = F_(pP, V, oN + oU), vND = F_(pP, V, oN + oD), vSU = F_(pP, V, oS + oU), vSD = F_(pP, V, oS + oD);
   const double mNdzw = muN * (wNU - wND), mSdzw = muS * (wSU - wSD);  // w_U - w_D at N, S

@@ -510,17 +510,22 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
       XNode gm1{}, gm2{};
       double fprev[5] = {0, 0, 0, 0, 0};
       XOwn ownPrev{};
-      constexpr int oN = HK, oU = 1;
+      // A single grid's columns keep the in-plane neighbours' velocities of the last three planes in registers: sixteen
+      // shared-memory loads fewer a node (Taylor-Green 256^3 2972 -> 2921 us per step, 128^3 432 -> 428; stages 1-3 only:
+      // 2934). An ensemble's columns, short of registers, would spill: 3975 -> 4150 us for the 64 members.
+      constexpr bool CARRY = !ENS;
+      Cross xW{}, xP{};
       // x-direction quantities of the column's node in staged plane slot (cX, pX): G of the node, and F of
       // the face towards the previous plane (a >= 1)
-      auto x_part = [&](int cX, int pX, bool face, XOwn& ownCur, XNode& gcur, double (&fcur)[5]) {
+      auto x_part = [&](int cX, int pX, bool face, XOwn& ownCur, XNode& gcur, double (&fcur)[5], Cross& xCur) {
         const double* cs = reinterpret_cast<const double*>(consBase + cX * CONS_SLOT);
         const double* ps = reinterpret_cast<const double*>(primBase + pX * PRIM_SLOT);
+        const CrossMem<HK, FS> xm{ps, cidx};
+        if constexpr (CARRY) xCur = xm.load();
         ownCur = XOwn{ps[5 * FS + cidx], ps[0 * FS + cidx], ps[1 * FS + cidx], ps[2 * FS + cidx], ps[4 * FS + cidx]};
         gcur = x_node(C, cs[1 * FS + cidx], cs[2 * FS + cidx], cs[3 * FS + cidx], cs[4 * FS + cidx], ownCur.u,
-                      ownCur.v, ownCur.w, ps[3 * FS + cidx], ownCur.mu,
-                      ps[1 * FS + cidx + oN] - ps[1 * FS + cidx - oN], ps[0 * FS + cidx + oN] - ps[0 * FS + cidx - oN],
-                      ps[2 * FS + cidx + oU] - ps[2 * FS + cidx - oU], ps[0 * FS + cidx + oU] - ps[0 * FS + cidx - oU]);
+                      ownCur.v, ownCur.w, ps[3 * FS + cidx], ownCur.mu, xm.vN() - xm.vS(), xm.uN() - xm.uS(),
+                      xm.wU() - xm.wD(), xm.uU() - xm.uD());
 #pragma unroll
         for (int f = 0; f < 5; ++f) fcur[f] = 0.0;
         if (face) x_face(C, ownPrev, ownCur, fcur);
@@ -538,7 +543,10 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
         XNode gcur;
         XOwn ownCur;
         double fcur[5];
-        x_part(cX, pX, a >= 1, ownCur, gcur, fcur);
+        Cross xCur;
+        x_part(cX, pX, a >= 1, ownCur, gcur, fcur, xCur);
+        xW = xP;
+        xP = xCur;
         if (a == 0) {  // plane i0-1: its conserved values have no other reader
           __syncwarp();
           if (lane == 0) mbar_arrive(&consEmpty[cX]);
@@ -568,7 +576,8 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
         XNode gcur;
         XOwn ownCur;
         double fcur[5];
-        x_part(cX, pX, true, ownCur, gcur, fcur);
+        Cross xCur;
+        x_part(cX, pX, true, ownCur, gcur, fcur, xCur);
         if constexpr (ENS) {
           if (!mbar_wait(&epiFull[se], (e / NE) & 1, abortFlag, lim)) {
             ok = false;
@@ -580,9 +589,16 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
         const uint8_t tc = (reinterpret_cast<const uint8_t*>(cP) + TYPE_OFF)[tcix];
         const bool valid = inTile && (tc & TYPE_MASK) == FLUID_INTERIOR;
         double kk5[5];
-        yz_part<HK, FS>(C, cP, reinterpret_cast<const double*>(primBase + pW * PRIM_SLOT),
-                        reinterpret_cast<const double*>(primBase + pR * PRIM_SLOT),
-                        reinterpret_cast<const double*>(primBase + pX * PRIM_SLOT), cidx, ownPrev, kk5);
+        const double* const pP = reinterpret_cast<const double*>(primBase + pR * PRIM_SLOT);
+        if constexpr (!CARRY) {
+          using X = CrossMem<HK, FS>;
+          yz_part<HK, FS>(C, cP, pP, X{reinterpret_cast<const double*>(primBase + pW * PRIM_SLOT), cidx}, X{pP, cidx},
+                          X{reinterpret_cast<const double*>(primBase + pX * PRIM_SLOT), cidx}, cidx, ownPrev, kk5);
+        } else {
+          yz_part<HK, FS>(C, cP, pP, xW, xP, xCur, cidx, ownPrev, kk5);
+          xW = xP;
+          xP = xCur;
+        }
 #pragma unroll
         for (int f = 0; f < 5; ++f) kk5[f] += (gcur.g[f] - gm2.g[f]) + (fcur[f] - fprev[f]);
         const double* ep = reinterpret_cast<const double*>(sm + OFF_EPI + se * EPI_SLOT);

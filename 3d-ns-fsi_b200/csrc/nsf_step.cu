@@ -181,7 +181,8 @@ __device__ __forceinline__ void stage_tile(const Grid& G, const StepCtl& c, int 
       double f[5], kk[5];
       x_part(a + 2, true, own, g, f);
       const double* pP = sm + (a + 1) * PS;
-      yz_part<HK, FS>(C, pP + 5 * FS, pP - PS, pP, pP + PS, cidx, ownPrev, kk);
+      using X = CrossMem<HK, FS>;
+      yz_part<HK, FS>(C, pP + 5 * FS, pP, X{pP - PS, cidx}, X{pP, cidx}, X{pP + PS, cidx}, cidx, ownPrev, kk);
 #pragma unroll
       for (int e = 0; e < 5; ++e) kk[e] += (g.g[e] - gm2.g[e]) + (f[e] - fprev[e]);
       const bool valid = (tc & TYPE_MASK) == FLUID_INTERIOR;
