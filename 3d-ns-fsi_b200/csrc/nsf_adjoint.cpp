@@ -712,7 +712,7 @@ nsf_status enqueue_adjoint_kernels(nsf_solver* s, AdjCtx* a, const StepCtl& R, b
     P.timeout = a->dTimeout;
     launch_adj_bc(G, P, q, nSM, st);
     mark(PH_BC);
-    launch_adj_rhs(s->dGrid, G, A, a->tmpLam, a->tmpV, nSM, st);
+    launch_adj_rhs(s->dGrid, G, A, a->tmpLam, a->tmpV, st);
     mark(PH_RHS);
   }
   if (R.filterNow) {

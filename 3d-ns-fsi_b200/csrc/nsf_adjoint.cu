@@ -730,7 +730,7 @@ int adj_kernels_init() {
   return int(cudaFuncSetAttribute(k_adj_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM));
 }
 
-void launch_adj_rhs(const Grid* dg, const Grid& hg, const AdjPtrs& A, const double* lam, const double* V, int nSM,
+void launch_adj_rhs(const Grid* dg, const Grid& hg, const AdjPtrs& A, const double* lam, const double* V,
                     void* stream) {
   const int tiles = ((hg.NJ + RT_J - 1) / RT_J) * ((hg.NK + RT_K - 1) / RT_K);
   k_adj_rhs<<<dim3(tiles, (hg.NI + RT_L - 1) / RT_L), RT_THREADS, RT_SMEM, static_cast<cudaStream_t>(stream)>>>(

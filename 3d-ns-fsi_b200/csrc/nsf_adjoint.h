@@ -68,7 +68,7 @@ struct AdjBcParams {
 void launch_adj_bc(const Grid& hg, const AdjBcParams& P, int s, int nSM, void* stream);
 // The transposed RHS (gather) and the chain rule through the primitives into the stage input's adjoints,
 // from launch_adj_bc's lam and V.
-void launch_adj_rhs(const Grid* dg, const Grid& hg, const AdjPtrs& A, const double* lam, const double* V, int nSM,
+void launch_adj_rhs(const Grid* dg, const Grid& hg, const AdjPtrs& A, const double* lam, const double* V,
                     void* stream);
 // Kernel attributes (shared-memory size of the transposed RHS); call once before the first launch.
 int adj_kernels_init();

@@ -1,5 +1,8 @@
-// CUDA kernels (sm_100a, FP64) of the RK4 time-marching path. One RK4 step (Solver::marchTimeStep,
-// Solver.cpp:130-167) is the launch sequence enqueue_step() builds:
+// CUDA kernels (sm_100a, FP64) of the RK4 time-marching path. Grids up to kStepMaxNodes (nsf_capi.cpp) run whole steps
+// in one kernel (nsf_step.cu); of the others one RK4 step (Solver::marchTimeStep, Solver.cpp:130-167) is the launch
+// sequence enqueue_step() builds, in which k_bc takes everything between two stage kernels, and the end of the step, in
+// one launch; the kernels it stands for run by themselves where a boundary plan is not built or the adjoint's
+// recomputation must read the state between them:
 //
 //   k_prologue            stop criterion, filter decision, buffer roles        (Solver.cpp:133-135)
 //   k_density_filter      global 2nd-order density filter, rare              (Mesh.cpp:108-140)
@@ -43,7 +46,6 @@ __global__ void k_density_filter(const Grid* __restrict__ grids) {
   for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < g->N; n += (long long)gridDim.x * blockDim.x)
     density_filter_node(*g, c, n);
 }
-
 
 __global__ void k_solid_copy(const Grid* __restrict__ grids, int s) {
   const Grid* g = grids + blockIdx.y;
