@@ -1,5 +1,6 @@
 // C ABI implementation (include/nsfsi.h): the solver handle, device residency of all fields, the
-// device-side lists built from the host setup, and one captured CUDA graph per RK4 step.
+// device-side lists built from the host setup, and the queueing of steps: one cooperative launch for up to 64 steps of a
+// small grid, one captured CUDA graph per RK4 step of the others.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -58,6 +59,7 @@ Consts make_consts(const nsf_config& c, const HostSetup& s) {
   K.pr = c.pr;
   K.re = c.re;
   K.sc1 = 1 + c.sutherlands_c2 / c.t0;
+  K.muA = c.re / K.sc1;
   K.pf = 1 / (K.gm1 * c.pr);
   K.h0 = 1. / (c.gamma - 1);
   K.vmod = std::max(4. / 3, c.gamma / c.pr);
