@@ -47,11 +47,11 @@ constexpr int NPRIM = 6;                          // staged primitive fields: u,
 constexpr int MAP_CONS = 0, MAP_EPI = 15, MAP_ACC = 30, MAP_TYPE = 35, NMAPS = 36;
 constexpr long long WAIT_LIMIT = 1ll << 22;  // default polls before a wait is declared failed (StepCtl::waitLimit)
 // Register split (setmaxnreg): the launch gives every thread 168 registers (384 x 168 = 64,512); a split must not
-// exceed that total. Warpgroup 0 gets 88 and the column warpgroups 208: 128 x 88 + 256 x 208 = 64,512. With
-// near-body filter nodes (FLT) the staging of a body's planes needs more, 128 x 104 + 256 x 200 = 64,512 (sphere
-// 128^3: 485 us per step against 494 with 88 / 208); an ensemble's stage 4 stays at 88 / 208, since its columns
-// spill below (64 members: 3990 us per step, 4003 with 104 / 200, 4047 with 72 / 216).
-constexpr int REG_LAUNCH = 168, REG_LOW = 88, REG_HIGH = 208, REG_LOW_FLT = 104, REG_HIGH_FLT = 200;
+// exceed that total. Warpgroup 0 gets 104, which the staging of a body's planes needs, and the column warpgroups 200:
+// 128 x 104 + 256 x 200 = 64,512 (sphere 128^3: 485 us per step against 494 with 88 / 208, grids without bodies the
+// same by either); an ensemble's stage 4, whose columns spill below, has 88 / 208 (64 members: 3990 us per step, 4003
+// with 104 / 200, 4047 with 72 / 216).
+constexpr int REG_LAUNCH = 168, REG_LOW = 104, REG_HIGH = 200, REG_LOW_ENS4 = 88, REG_HIGH_ENS4 = 208;
 
 constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -102,7 +102,7 @@ struct Tile {
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
   static_assert(NSTAGE * NPASS >= HP && NSTAGE * (NPASS - 1) <= HP && NPASS % 2 == 0, "four staging passes cover a plane");
   static_assert(128 * REG_LOW + NCOL * REG_HIGH <= NTHREADS * REG_LAUNCH, "register split exceeds the launch total");
-  static_assert(128 * REG_LOW_FLT + NCOL * REG_HIGH_FLT <= NTHREADS * REG_LAUNCH, "register split exceeds the launch total");
+  static_assert(128 * REG_LOW_ENS4 + NCOL * REG_HIGH_ENS4 <= NTHREADS * REG_LAUNCH, "register split exceeds the launch total");
 };
 }  // namespace ws
 
@@ -167,12 +167,12 @@ __device__ __forceinline__ void reg_alloc() {
 // only stage with dt maxima, change norms and the NaN check; mode 1 carries none of their registers). The
 // single grid runs mode 0 for stages 1-3 and mode 2 for stage 4, an ensemble modes 1 and 2: the fastest
 // pairing measured (mode 1 frees registers an ensemble needs, but its schedule is slower for one grid).
-// FLT: the grid has near-body filter nodes. Without them the staging looks at no node type; with them it takes an
-// item that has any (StageItem::f0 .. f1) through a second copy of its loop. The staging warps pace the kernel: in
-// one loop for both, a pair of filter nodes held their warp up for four trips to L2 in a row, and any work added
-// for it slowed every grid by 5-7 %. Measured (us per step, before / now): sphere 96^3 379 / 293, sphere 128^3
-// 579 / 485, 16 spheres 256x128x128 980 / 866, the 64-member ensemble 4069 / 3990, Taylor-Green 128^3 440 / 431.
-template <int TK_, int TJ_, bool ENS, int MODE, bool FLT>
+// The staging takes an item that has near-body filter nodes in its planes f0 .. f1 through a second copy of its loop;
+// the first looks at no node type. The staging warps pace the kernel: in one loop for both, a pair of filter nodes
+// held their warp up for four trips to L2 in a row, and any work added for it slowed every grid by 5-7 %. Measured (us
+// per step, one loop / two): sphere 96^3 379 / 293, sphere 128^3 579 / 485, 16 spheres 256x128x128 980 / 866, the
+// 64-member ensemble 4069 / 3990, Taylor-Green 128^3 440 / 431.
+template <int TK_, int TJ_, bool ENS, int MODE>
 __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
     k_stage_ws(const __grid_constant__ Grid G0, const Grid* __restrict__ grids, const StageItem* __restrict__ items,
                const int* __restrict__ ctaStart, int s) {
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
   auto skip = [&](const StageItem& w) { return ENS && !ctl_of(grid_of(w)).active; };
 
   if (warp < 4) {
-    reg_dealloc<FLT && !(ENS && MODE == 2) ? REG_LOW_FLT : REG_LOW>();
+    reg_dealloc<ENS && MODE == 2 ? REG_LOW_ENS4 : REG_LOW>();
     if (warp == 0) {
       // ------------------------------------------------------------------ producer (one thread)
       if (lane == 0) {
@@ -432,14 +432,14 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
             if (lane == 0) mbar_arrive(&primFull[ps]);
           }
         };
-        if (FLT && G.nFilter > 0 && w.f0 <= w.f1)
+        if (G.nFilter > 0 && w.f0 <= w.f1)
           stage_planes(std::true_type{});
         else
           stage_planes(std::false_type{});
       }
     }
   } else {
-    reg_alloc<FLT && !(ENS && MODE == 2) ? REG_HIGH_FLT : REG_HIGH>();
+    reg_alloc<ENS && MODE == 2 ? REG_HIGH_ENS4 : REG_HIGH>();
     // -------------------------------------------------------------------- columns (warpgroups 1-2)
     const int ct = tid - 128, tx = ct % TK, ty = ct / TK;
     const int cidx = (ty + 1) * HK + (tx + 1);   // this column's node in a staged plane
@@ -510,10 +510,10 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
       XNode gm1{}, gm2{};
       double fprev[5] = {0, 0, 0, 0, 0};
       XOwn ownPrev{};
-      // A single grid's columns keep the in-plane neighbours' velocities of the last three planes in registers: sixteen
-      // shared-memory loads fewer a node (Taylor-Green 256^3 2972 -> 2921 us per step, 128^3 432 -> 428; stages 1-3 only:
-      // 2934). An ensemble's columns, short of registers, would spill: 3975 -> 4150 us for the 64 members.
-      constexpr bool CARRY = !ENS;
+      // The columns keep the in-plane neighbours' velocities of the last three planes in registers: sixteen shared-memory
+      // loads fewer a node (Taylor-Green 256^3 2972 -> 2921 us per step, 128^3 432 -> 428, the 64-member ensemble 3693 ->
+      // 3667). An ensemble's stage 4 has no registers left for them.
+      constexpr bool CARRY = !ENS || MODE == 1;
       Cross xW{}, xP{};
       // x-direction quantities of the column's node in staged plane slot (cX, pX): G of the node, and F of
       // the face towards the previous plane (a >= 1)
@@ -729,9 +729,8 @@ namespace {
 struct VariantInfo {
   int tk, tj, threads, typeBoxW;
   size_t smem;
-  // single grid: stages 1-3 (mode 0), stage 4 (mode 2); the same with near-body filter nodes; an ensemble's stages
-  // 1-3 (mode 1), stage 4 (mode 2)
-  const void* fn[6];
+  // single grid: stages 1-3 (mode 0), stage 4 (mode 2); an ensemble's stages 1-3 (mode 1), stage 4 (mode 2)
+  const void* fn[4];
 };
 template <int TK, int TJ>
 VariantInfo variant_info() {
@@ -741,12 +740,10 @@ VariantInfo variant_info() {
                      TL::NTHREADS,
                      TL::TYW,
                      TL::SMEM,
-                     {reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 0, false>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 2, false>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 0, true>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 2, true>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 1, true>),
-                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 2, true>)}};
+                     {reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 0>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, false, 2>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 1>),
+                      reinterpret_cast<const void*>(&k_stage_ws<TK, TJ, true, 2>)}};
 }
 VariantInfo info(int v) { return v == STAGE_TILE_16x16 ? variant_info<16, 16>() : variant_info<32, 8>(); }
 
@@ -757,15 +754,10 @@ void launch_variant(const Grid& hg, const Grid* dGrids, const LaunchPlan& L, int
   auto go = [&](auto kernel) {
     kernel<<<L.stageBlocks, TL::NTHREADS, TL::SMEM, st>>>(hg, dGrids, L.items, L.ctaStart, s);
   };
-  constexpr bool plain = ENS;  // a grid without filter nodes runs FLT = ENS
-  if (L.hasFilter && s == 3)
-    go(k_stage_ws<TK, TJ, ENS, 2, true>);
-  else if (L.hasFilter)
-    go(k_stage_ws<TK, TJ, ENS, early, true>);
-  else if (s == 3)
-    go(k_stage_ws<TK, TJ, ENS, 2, plain>);
+  if (s == 3)
+    go(k_stage_ws<TK, TJ, ENS, 2>);
   else
-    go(k_stage_ws<TK, TJ, ENS, early, plain>);
+    go(k_stage_ws<TK, TJ, ENS, early>);
 }
 }  // namespace
 
@@ -802,7 +794,7 @@ int stage_launch_registers(int v) {
 }
 bool stage_register_split_ok(int v) {
   const int r = stage_launch_registers(v);
-  const int need = std::max(128 * ws::REG_LOW + 256 * ws::REG_HIGH, 128 * ws::REG_LOW_FLT + 256 * ws::REG_HIGH_FLT);
+  const int need = std::max(128 * ws::REG_LOW + 256 * ws::REG_HIGH, 128 * ws::REG_LOW_ENS4 + 256 * ws::REG_HIGH_ENS4);
   return r > 0 && need <= info(v).threads * r;
 }
 void launch_stage(const Grid& hg, const LaunchPlan& L, int s, void* stream) {
