@@ -631,14 +631,14 @@ nsf_status build_device(nsf_solver* s) {
   }
   // Small grids: the whole-step kernel (its boundary work needs the fused plan above). The line lies where a step
   // of the launch sequence costs as much (us per step, graph / whole-step kernel, one B200): Taylor-Green 64^3
-  // 110 / 101, 80^3 188 / 170, 88^3 212 / 245; channel with a sphere 32^3 102 / 57, 48^3 130 / 72, 80^3 255 / 198.
+  // 104 / 100, 80^3 177 / 167, 84^3 193 / 228; channel with a sphere 64^3 142 / 118, 80^3 226 / 190, 88^3 263 / 269.
   // A requested tile shape (ensemble members, the tuner, NSF_STAGE_TILE) means the streaming stage kernel.
   constexpr size_t kStepMaxNodes = 550000;
   if (!s->grouped && s->tileRequest < 0 && !std::getenv("NSF_STAGE_TILE") && L.bcBlocks > 0 && N <= kStepMaxNodes) {
     const StepChoice ch = step_choose(G.NI, G.NJ, G.NK, s->nSM);
     const StepShape t = step_shape(ch.shape);
     const size_t smem = step_smem_bytes(ch.shape, ch.planes, L.bcLevels);
-    CK(cudaError_t(step_configure(ch.shape, smem)));
+    CK(cudaError_t(step_configure(ch.shape)));
     BcFlat fl;
     bc_flatten({&s->bcLevels}, fl);
     const int warps = int(std::min<long long>((fl.maxWork + 31) / 32, s->nSM));

@@ -259,7 +259,7 @@ struct StepChoice {
 StepShape step_shape(int shape);
 size_t step_smem_bytes(int shape, int planes, int levels);
 StepChoice step_choose(int NI, int NJ, int NK, int nSM);
-int step_configure(int shape, size_t smem);
+int step_configure(int shape);
 int step_capacity(int shape, size_t smem, int nSM);
 // What the steps leave for the discrete adjoint (nsf_adjoint.cpp), or stage == NULL: per step one set of values, set
 // (time level mod nSets) at stage + set * setWords and result + set * setWords. A set holds, per stage s at s * perStage,

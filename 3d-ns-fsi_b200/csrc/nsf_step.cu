@@ -454,11 +454,19 @@ StepChoice step_choose(int NI, int NJ, int NK, int nSM) {
   return best;
 }
 
-int step_configure(int shape, size_t smem) {
-  cudaError_t e = cudaSuccess;
-  for (bool tape : {false, true})
+// The attribute belongs to the function, not to a handle: it is set to all a block can have, whatever the handle's
+// plan takes, so that a handle created later does not take it below what an earlier one launches with.
+int step_configure(int shape) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  for (bool tape : {false, true}) {
+    cudaFuncAttributes a{};
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel_of(shape, tape));
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kernel_of(shape, tape), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      e = cudaFuncSetAttribute(kernel_of(shape, tape), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               most - int(a.sharedSizeBytes));
+  }
   return int(e);
 }
 

@@ -108,3 +108,22 @@ def test_two_solvers_side_by_side():
         for s, ref in ((a, alone[0]), (b, alone[1])):
             s.sync()
             assert np.array_equal(s.download(), ref, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flow,first,second", [("tgv", (81, 80, 82), (19, 11, 19)), ("shipped", (161, 83, 3), (21, 12, 3)),
+                                               ("sphere", (64, 60, 62), (30, 20, 20))], ids=["tgv", "thin", "sphere"])
+def test_a_later_smaller_handle_leaves_an_earlier_one_alone(flow, first, second):
+    """The kernel's shared-memory limit is a property of the function: a handle whose plan takes less, created after
+    one whose plan takes more, must not lower it (and the other way round)."""
+    big, small = config(flow, first, 3), config(flow, second, 3)
+    with nsfsi.Solver(big) as s:
+        s.march(3)
+        ref = s.download()
+    with nsfsi.Solver(big) as a, nsfsi.Solver(small) as b:
+        a.march(3)
+        b.march(3)
+        a.sync()
+        b.sync()
+        assert a.launches_per_step() == b.launches_per_step() == 1
+        assert np.array_equal(a.download(), ref, equal_nan=True)
