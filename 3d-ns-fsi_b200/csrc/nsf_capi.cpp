@@ -59,7 +59,9 @@ Consts make_consts(const nsf_config& c, const HostSetup& s) {
   K.pr = c.pr;
   K.re = c.re;
   K.sc1 = 1 + c.sutherlands_c2 / c.t0;
-  K.muA = c.re / K.sc1;
+  // mu_nr squares re (1 + T / sc1): a Reynolds number beyond 1e100 (a viscosity of none) must not overflow there
+  K.muRe = std::copysign(std::min(std::max(std::fabs(c.re), 1e-100), 1e100), c.re);
+  K.muA = K.muRe / std::copysign(std::max(std::fabs(K.sc1), 1e-40), K.sc1);
   K.pf = 1 / (K.gm1 * c.pr);
   K.h0 = 1. / (c.gamma - 1);
   K.vmod = std::max(4. / 3, c.gamma / c.pr);

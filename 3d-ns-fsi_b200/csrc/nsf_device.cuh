@@ -27,7 +27,7 @@ struct Consts {
   double gamma, gm1, pr, re, sc1, pf, h0, vmod, convLim, viscLim, m0, tEnd;
   double dx, dy, dz, dxdydz;
   double invD2;  // 1/dx^2 + 1/dy^2 + 1/dz^2
-  double muA;    // re / sc1 (mu_nr)
+  double muRe, muA;  // re and re / sc1, kept where mu_nr can square them
   // continuity / inviscid: -1/(2d)
   double ax, ay, az;
   // x-momentum: 2/(3dx^2), 1/(2dy^2), 1/(2dz^2), -1/(6dydx), 1/(4dxdy), -1/(6dzdx), 1/(4dxdz)

@@ -17,7 +17,7 @@ struct Prim {
 
 // The constants prims_of_nr reads, small enough to keep in registers.
 struct ThermoConsts {
-  double gamma, gm1, muA, re, pf;
+  double gamma, gm1, muA, muRe, pf;
 };
 
 __device__ __forceinline__ Prim prims_of(const Consts& C, double rho, double ru, double rv, double rw, double rE) {
@@ -57,13 +57,13 @@ __device__ __forceinline__ double sqrt_nr(double a) {
   return fma(fma(-s, s, a), 0.5 * r, s);
 }
 
-// Sutherland's viscosity x sqrt(x) sc1 / (re (T + sc1)), x = 1 + T, as x^2 / sqrt(x d^2) with d = re + T re/sc1 (C.muA =
-// re/sc1), with d's sign: one Newton-Raphson inverse square root in place of a square root and a reciprocal, twelve FP64
+// Sutherland's viscosity x sqrt(x) sc1 / (re (T + sc1)), x = 1 + T, as x^2 / sqrt(x d^2) with d = re + T re/sc1 (C.muRe,
+// C.muA), with d's sign: one Newton-Raphson inverse square root in place of a square root and a reciprocal, twelve FP64
 // operations in place of twenty. The last iteration is written as a correction of r, which keeps its rounding out of the
 // result: rms error 1.21-1.29e-16 over |T| <= 0.2 (the quotient form: 1.31-1.35e-16), largest 5.6e-16 (5.7e-16).
 template <class CT>
 __device__ __forceinline__ double mu_nr(const CT& C, double x, double T) {
-  const double d = fma(T, C.muA, C.re);
+  const double d = fma(T, C.muA, C.muRe);
   const double z = (x * d) * d;
   double r;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(z));

@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(ws::Tile<TK_, TJ_>::NTHREADS, 1)
         const StageItem w = items[it];
         if (skip(w)) continue;
         const Grid& G = grid_of(w);
-        const ThermoConsts C{G.C.gamma, G.C.gm1, G.C.muA, G.C.re, G.C.pf};
+        const ThermoConsts C{G.C.gamma, G.C.gm1, G.C.muA, G.C.muRe, G.C.pf};
         const double* __restrict__ fpre = G.fpre;
         const int* const fidx = G.fidx;
         const long long sIs = G.sI, sJs = G.sJ;

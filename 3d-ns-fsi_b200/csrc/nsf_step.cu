@@ -82,7 +82,7 @@ __device__ __forceinline__ void stage_tile(const Grid& G, const StepCtl& c, int 
     const double* const q2 = c.I[s][2];
     const double* const q3 = c.I[s][3];
     const double* const q4 = c.I[s][4];
-    const ThermoConsts TC{C.gamma, C.gm1, C.muA, C.re, C.pf};
+    const ThermoConsts TC{C.gamma, C.gm1, C.muA, C.muRe, C.pf};
     constexpr int U = 4;  // nodes a thread loads before it computes: their loads and reciprocal chains overlap
     const int total = (L + 2) * HP;
 #pragma unroll 1

@@ -127,3 +127,22 @@ def test_a_later_smaller_handle_leaves_an_earlier_one_alone(flow, first, second)
         b.sync()
         assert a.launches_per_step() == b.launches_per_step() == 1
         assert np.array_equal(a.download(), ref, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile", [None, "32x8"], ids=["whole_step", "streaming"])
+def test_reynolds_numbers_without_viscosity(tile, monkeypatch):
+    """The viscosity squares the Reynolds number: values whose square overflows run as ones that only make the viscous
+    terms vanish against the last bit of the others."""
+    if tile:
+        monkeypatch.setenv("NSF_STAGE_TILE", tile)
+    fields = []
+    for re in (1e60, 1e200, 1e300):
+        cfg = config("tgv", (24, 21, 23), 5)
+        cfg.re = re
+        with nsfsi.Solver(cfg) as s:
+            s.march(5)
+            s.sync()
+            fields.append(s.download(range(5)))
+    assert np.all(np.isfinite(fields[0]))
+    assert np.array_equal(fields[0], fields[1]) and np.array_equal(fields[0], fields[2])
