@@ -744,10 +744,34 @@ double nsf_initial_dt(const nsf_config& c, const nsf::HostSetup& S, const std::v
   return initial_dt(c, S, cons, prim);
 }
 
+// The handle's device while in scope: a launch, unlike a copy, is refused on a stream of another device than the
+// calling thread's. The thread's own device is put back, so reading a handle's state does not change it.
+namespace {
+struct DeviceScope {
+  int before = -1;
+  cudaError_t err;
+  explicit DeviceScope(int device) {
+    int now = -1;
+    err = cudaGetDevice(&now);
+    if (err == cudaSuccess && now != device) {
+      err = cudaSetDevice(device);
+      if (err == cudaSuccess) before = now;
+    }
+  }
+  ~DeviceScope() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+  DeviceScope(const DeviceScope&) = delete;
+  DeviceScope& operator=(const DeviceScope&) = delete;
+};
+}  // namespace
+
 // The control block after everything queued on the solver's stream: written into page-locked host memory by a
 // kernel queued behind that work, then one wait. (A copy would queue on the device's download engine behind a
 // snapshot still travelling to the host: 805 MB, 16 ms, for the 256^3 Taylor-Green case's saved fields.)
 static nsf_status read_ctl(nsf_solver* s, StepCtl* out) {
+  const DeviceScope on(s->device);
+  CK(on.err);
   if (!s->hCtl) CK(cudaHostAlloc(&s->hCtl, sizeof(StepCtl), cudaHostAllocMapped));
   void* dev = nullptr;
   CK(cudaHostGetDevicePointer(&dev, s->hCtl, 0));
