@@ -356,6 +356,9 @@ nsf_status reset(nsf_solver* s, AdjCtx* a) {
   CKA(cudaMemcpyAsync(G.bufs[0][0], a->dU0, 5 * N * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
   CKA(cudaMemsetAsync(G.bufs[1][0], 0, 15 * N * sizeof(double), s->stream));  // buffers 1, 2 and the accumulator
   launch_fpre_init(s->dGrid, G.nFilter, G.bufs[0][0], G.bufs[0][4], s->nSM, s->stream);
+  // The control block takes its flags with it, a give-up of the whole-step kernel's barrier among them; such a run may
+  // have left the barrier's counter at no multiple of the block count, which the next launch takes it to be.
+  if (s->plan.stepSync) CKA(cudaMemsetAsync(s->plan.stepSync, 0, sizeof *s->plan.stepSync, s->stream));
   StepCtl c = s->ctlInit;
   if (a->haveDt) c.dt = a->dts[0];
   CKA(cudaMemcpyAsync(s->dCtl, &c, sizeof c, cudaMemcpyHostToDevice, s->stream));

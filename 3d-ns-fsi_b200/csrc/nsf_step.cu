@@ -309,7 +309,8 @@ __global__ void __launch_bounds__(NT, 1) k_step(const __grid_constant__ Grid G0,
   // warps are numbered across the blocks, so that a short list of boundary items spreads over all SMs
   const int gtid = (warp * int(gridDim.x) + int(blockIdx.x)) * 32 + lane, nthr = int(gridDim.x) * NT;
   // every earlier launch left the counter at a multiple of the block count, and the first barrier cannot pass
-  // before this block has arrived, so the value at the launch is the counter rounded down to a multiple
+  // before this block has arrived, so the value at the launch is the counter rounded down to a multiple. (A launch
+  // whose barrier gave up may not have; its flag stays until the control block is reset, and the counter with it.)
   StepBarrier bar{P.sync, tid == 0 ? ld_acquire(P.sync) / gridDim.x * gridDim.x : 0ull, &gc->timeout, false};
   auto barrier = [&] { bar.wait(cs); };
   // the first boundary item each thread has in the first kStash levels, resolved once for the whole launch
