@@ -18,9 +18,9 @@
 // A group lives in one process or spans several (one GPU each, nsf_slab_group_create_ranks): rank r holds
 // the consecutive slabs p with p * world / P == r. Each process's slabs share one device and one stream,
 // and a step is one CUDA graph that treats them as an ensemble's members: one stage launch over the union of their
-// work items (or one per slab, kSharedStageCost) and one boundary launch (Taylor-Green 96^3 in two slabs: 41 launches
-// and 410 us per step before, 303 us now; 64^3 in three 339, 162). A
-// transfer within the process copies the plane from slab to slab (the buffers each step's roles select are read on
+// work items (or one per slab, kSharedStageCost) and one boundary launch (or one per slab, where more slabs than
+// resident blocks share the process; Taylor-Green 96^3 in two slabs: 41 launches and 410 us per step before, 303 us
+// now; 64^3 in three 339, 162). A transfer within the process copies the plane from slab to slab (the buffers each step's roles select are read on
 // the device); across processes it is packed into a staging buffer, moved by NCCL send/recv (captured in the graph)
 // and unpacked on the receiving side. The global reductions gather every slab's partials (NCCL all-gather
 // across processes) and combine them in slab order, so every process computes the same dt and norms.
@@ -58,6 +58,7 @@ struct nsf_slab_group {
   bool xPeriodic = false;
   LaunchPlan plan{};               // one stage and one boundary launch over this process's slabs
   bool oneStage = true;            // false: a stage launch per slab (see kSharedStageCost)
+  bool oneBoundary = true;         // false: a boundary launch per slab (they do not fit one launch)
   std::vector<Grid> hGrids;        // this process's slabs' grids with the plan's norm slots
   Grid* dGrids = nullptr;          // the same on the device
   double* dPart = nullptr;         // [9 x local slabs] this process's slab partials
@@ -276,12 +277,14 @@ nsf_status build_group(nsf_slab_group* g, int P, const void* ncclId) {
     return st;
   double apart = 0;
   for (nsf_solver* s : g->slabs) apart += s->plan.stageSpan + kStageLaunchPlanes;
-  g->oneStage = kSharedStageCost * g->plan.stageSpan < apart;
+  // the boundary launch needs all its blocks resident, at least one per slab: a process with more slabs than that
+  // (592 on a B200) runs each slab's own launches
+  g->oneBoundary = g->plan.bcBlocks > 0;
+  g->oneStage = g->oneBoundary && kSharedStageCost * g->plan.stageSpan < apart;
   if (!g->oneStage) {  // each slab's own stage launches write its own norm slots
     for (size_t l = 0; l < g->slabs.size(); ++l) g->hGrids[l] = g->slabs[l]->hGrid;
     CKG(cudaMemcpy(g->dGrids, g->hGrids.data(), g->hGrids.size() * sizeof(Grid), cudaMemcpyHostToDevice));
   }
-  if (g->plan.bcBlocks <= 0) return gfail(g, NSF_ERR_CUDA, "the slabs do not fit one launch of the boundary kernel");
   if ((st = galloc(g, &g->dRed, 9)) != NSF_OK) return st;
   if ((st = galloc(g, &g->dPart, size_t(9) * size_t(g->maxLocal))) != NSF_OK) return st;
   CKG(cudaMemset(g->dPart, 0, size_t(9) * size_t(g->maxLocal) * sizeof(double)));
@@ -395,7 +398,10 @@ nsf_status build_group(nsf_slab_group* g, int P, const void* ncclId) {
       }
     }
     exchange(1, q);
-    launches += launch_bc_part(g->dGrids, nLocal, g->plan, q, false, g->stream);
+    if (g->oneBoundary)
+      launches += launch_bc_part(g->dGrids, nLocal, g->plan, q, false, g->stream);
+    else
+      for (nsf_solver* s : g->slabs) launches += launch_bc_part(s->dGrid, 1, s->plan, q, false, g->stream);
     exchange(0, q);
   }
   if (useNccl) {
