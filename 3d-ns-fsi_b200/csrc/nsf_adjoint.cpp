@@ -1056,7 +1056,7 @@ nsf_status nsf_adj_backward(nsf_solver* s, double dJ, double* g_inflow, double* 
   int adjTimeout = 0;
   CKA(cudaMemcpy(&ctl, s->dCtl, sizeof ctl, cudaMemcpyDeviceToHost));
   CKA(cudaMemcpy(&adjTimeout, a->dTimeout, sizeof adjTimeout, cudaMemcpyDeviceToHost));
-  if (ctl.timeout) return fail(s, NSF_ERR_TIMEOUT, "a bounded wait in the stage kernel gave up during the adjoint");
+  if (ctl.timeout) return fail(s, NSF_ERR_TIMEOUT, "a bounded wait of the step's kernels gave up during the adjoint");
   if (adjTimeout) return fail(s, NSF_ERR_TIMEOUT, "a grid barrier of the adjoint boundary kernel gave up");
   const size_t hp = S.NK * sizeof(double), dp = size_t(G.NKp) * sizeof(double);
   if (g_u0) {

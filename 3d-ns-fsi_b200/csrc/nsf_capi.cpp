@@ -891,7 +891,7 @@ nsf_status nsf_sync(nsf_solver* s) {
   const nsf_status st = read_ctl(s, &ctl);
   if (st != NSF_OK) return st;
   if (ctl.timeout) {
-    s->err = "a bounded wait in the stage kernel gave up; results of the affected steps are invalid";
+    s->err = "a bounded wait of the step's kernels gave up; results of the affected steps are invalid";
     return NSF_ERR_TIMEOUT;
   }
   if (ctl.nonFinite) {

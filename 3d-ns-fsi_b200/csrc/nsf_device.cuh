@@ -53,9 +53,9 @@ struct StepCtl {
   unsigned long long level;  // timeLevel
   int perm[5][3];         // per field: physical buffer of [cons, old, scratch]
   int nonFinite;          // sticky NaN/Inf flag (Mesh::checkFinity)
-  // Test support for the bounded waits of the stage kernel (left at 0 in normal runs): withhold = 1 makes
-  // its producer issue no epilogue-ring load, so the column warps' waits run out; waitLimit = polls
-  // before a wait gives up (0: the kernel's default).
+  // Test support for the bounded waits (left at 0 in normal runs): with withhold = 1 the stage kernel's producer issues
+  // no epilogue-ring load, so the column warps' waits run out, and block 0 of the whole-step kernel does not arrive at
+  // its barriers; waitLimit = polls before a wait gives up (0: the kernel's default).
   int withhold;
   // per-step decisions (prologue)
   int active;             // 0: step is a no-op (end_time reached)

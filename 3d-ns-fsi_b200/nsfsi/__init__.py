@@ -299,8 +299,8 @@ class Solver:
         return snap
 
     def debug_wait_limit(self, polls=0, withhold_epilogue=False):
-        """Test support: the stage kernel's wait limit in polls (0: default) and the switch that withholds
-        its epilogue loads (nsf_debug_wait_limit)."""
+        """Test support: the wait limit in polls (0: default) and the switch that withholds the stage kernel's epilogue
+        loads or, on a small grid, a block's arrivals at the whole-step kernel's barrier (nsf_debug_wait_limit)."""
         self._check(lib().nsf_debug_wait_limit(self.h, polls, 1 if withhold_epilogue else 0))
 
     def upload_conserved(self, u5):

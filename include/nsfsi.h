@@ -330,11 +330,12 @@ nsf_status nsf_adj_profile_step(nsf_solver* s, uint64_t step, double* ms);
  * = the refined reciprocal, the IEEE 1/x, the refined square root, the IEEE sqrt(x). */
 nsf_status nsf_math_selftest(int32_t device, uint64_t n, const double* x, double* out);
 
-/* Test support for the bounded waits (no counterpart in the reference): every wait of the stage
- * kernel gives up after `polls` polls (0 restores the default of 2^22), and withhold_epilogue = 1 makes
- * the kernel's producer issue none of its epilogue loads, so the waits for them run out. A step that
- * ran with the switch on is invalid: nsf_sync then returns NSF_ERR_TIMEOUT and the handle should be
- * destroyed. Synchronises. */
+/* Test support for the bounded waits (no counterpart in the reference): a wait gives up after `polls` polls (0
+ * restores the default: 2^22 in the stage kernel, 2^24 at a barrier of the whole-step kernel of small grids), and
+ * withhold_epilogue = 1 withholds what the kernel waits for: the stage kernel's producer issues none of its epilogue
+ * loads, a whole-step launch's first block none of its barrier arrivals. A step that ran with the switch on is
+ * invalid: nsf_sync then returns NSF_ERR_TIMEOUT, and the handle should be destroyed (an adjoint run on it starts
+ * over from level 0 and is valid). Synchronises. */
 nsf_status nsf_debug_wait_limit(nsf_solver* s, uint64_t polls, int32_t withhold_epilogue);
 
 /* Text of the last error on this handle (static storage owned by the handle). */
