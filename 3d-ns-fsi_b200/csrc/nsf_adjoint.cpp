@@ -357,8 +357,9 @@ nsf_status reset(nsf_solver* s, AdjCtx* a) {
   CKA(cudaMemsetAsync(G.bufs[1][0], 0, 15 * N * sizeof(double), s->stream));  // buffers 1, 2 and the accumulator
   launch_fpre_init(s->dGrid, G.nFilter, G.bufs[0][0], G.bufs[0][4], s->nSM, s->stream);
   // The control block takes its flags with it, a give-up of the whole-step kernel's barrier among them; such a run may
-  // have left the barrier's counter at no multiple of the block count, which the next launch takes it to be.
-  if (s->plan.stepSync) CKA(cudaMemsetAsync(s->plan.stepSync, 0, sizeof *s->plan.stepSync, s->stream));
+  // have left a plan's barrier counter at no multiple of its block count, which the next launch takes it to be.
+  if (s->plan.stepSync)
+    CKA(cudaMemsetAsync(s->plan.stepSync, 0, STEP_WIDTHS * sizeof *s->plan.stepSync, s->stream));
   StepCtl c = s->ctlInit;
   if (a->haveDt) c.dt = a->dts[0];
   CKA(cudaMemcpyAsync(s->dCtl, &c, sizeof c, cudaMemcpyHostToDevice, s->stream));
@@ -520,7 +521,7 @@ enum TapeMode { TAPE_NONE, TAPE_FULL, TAPE_SEGMENTS };
 // The whole-step kernel records a step's set itself, except the planes before the edge conditions, which lie between its
 // phases (they are only kept where the inlet / outlet planes are not clean).
 bool step_kernel_tapes(const nsf_solver* s, const AdjCtx* a) {
-  return s->plan.stepBlocks > 0 && !(a->xInOut && !a->edgePlanesClean);
+  return s->plan.step[0].blocks > 0 && !(a->xInOut && !a->edgePlanesClean);
 }
 
 // Queues n steps of the forward run that record their tape sets.

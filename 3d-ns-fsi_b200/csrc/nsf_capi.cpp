@@ -1,5 +1,5 @@
 // C ABI implementation (include/nsfsi.h): the solver handle, device residency of all fields, the
-// device-side lists built from the host setup, and the queueing of steps: one cooperative launch for up to 64 steps of a
+// device-side lists built from the host setup, and the queueing of steps: one cooperative launch for up to 16 steps of a
 // small grid, one captured CUDA graph per RK4 step of the others.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -28,6 +29,9 @@ nsf_status cuda_fail(nsf_solver* s, cudaError_t e, const char* what) {
   s->err = std::string(what) + ": " + cudaGetErrorString(e);
   return NSF_ERR_CUDA;
 }
+// The largest grid (device nodes) whose steps run in the whole-step kernel (see build_device).
+constexpr size_t kStepMaxNodes = 550000;
+
 #define CK(call)                                              \
   do {                                                        \
     cudaError_t e_ = (call);                                  \
@@ -635,36 +639,51 @@ nsf_status build_device(nsf_solver* s) {
   // of the launch sequence costs as much (us per step, graph / whole-step kernel, one B200): Taylor-Green 64^3
   // 104 / 100, 80^3 177 / 167, 84^3 193 / 228; channel with a sphere 64^3 142 / 118, 80^3 226 / 190, 88^3 263 / 269.
   // A requested tile shape (ensemble members, the tuner, NSF_STAGE_TILE) means the streaming stage kernel.
-  constexpr size_t kStepMaxNodes = 550000;
   if (!s->grouped && s->tileRequest < 0 && !std::getenv("NSF_STAGE_TILE") && L.bcBlocks > 0 && N <= kStepMaxNodes) {
-    const StepChoice ch = step_choose(G.NI, G.NJ, G.NK, s->nSM);
-    const StepShape t = step_shape(ch.shape);
-    const size_t smem = step_smem_bytes(ch.shape, ch.planes, L.bcLevels);
-    CK(cudaError_t(step_configure(ch.shape)));
     BcFlat fl;
     bc_flatten({&s->bcLevels}, fl);
-    const int warps = int(std::min<long long>((fl.maxWork + 31) / 32, s->nSM));
-    const int blocks = std::min(std::max(ch.items, warps), step_capacity(ch.shape, smem, s->nSM));
-    if (blocks > 0) {
-      std::vector<StageItem> all, ordered;
+    std::vector<StageItem> items;  // the plans' lists, one after another
+    std::vector<int> start;
+    size_t itemsAt[STEP_WIDTHS] = {}, startAt[STEP_WIDTHS] = {}, partAt[STEP_WIDTHS] = {}, parts = 0;
+    for (int w = 0; w < STEP_WIDTHS; ++w) {
+      StepPlan& p = L.step[w];
+      const int nSM = std::max(1, s->nSM >> w);
+      const StepChoice ch = step_choose(G.NI, G.NJ, G.NK, nSM);
+      const StepShape t = step_shape(ch.shape);
+      CK(cudaError_t(step_configure(ch.shape)));
+      p.shape = ch.shape;
+      p.planes = ch.planes;
+      p.smem = step_smem_bytes(ch.shape, ch.planes, L.bcLevels);
+      const int warps = int(std::min<long long>((fl.maxWork + 31) / 32, nSM));
+      p.blocks = std::min(std::max(ch.items, warps), step_capacity(ch.shape, p.smem, nSM));
+      itemsAt[w] = items.size();
+      startAt[w] = start.size();
+      partAt[w] = parts;
+      parts += 9 * size_t(std::max(0, p.blocks));
+      std::vector<StageItem> all;
       for (int c0 = 1; c0 <= planes; c0 += ch.planes)
         for (int j0 = 1; j0 <= G.NJ - 2; j0 += t.tj)
           for (int k0 = 1; k0 <= G.NK - 2; k0 += t.tk)
             all.push_back(StageItem{j0, k0, c0, std::min(planes, c0 + ch.planes - 1), 0});
-      std::vector<int> start(1, 0);
-      for (int b = 0; b < blocks; ++b) {
-        for (size_t q = size_t(b); q < all.size(); q += size_t(blocks)) ordered.push_back(all[q]);
-        start.push_back(int(ordered.size()));
+      start.push_back(0);
+      for (int b = 0; b < p.blocks; ++b) {
+        for (size_t q = size_t(b); q < all.size(); q += size_t(p.blocks)) items.push_back(all[q]);
+        start.push_back(int(items.size() - itemsAt[w]));
       }
-      if ((st = upload(s, &L.stepItems, ordered)) != NSF_OK) return st;
-      if ((st = upload(s, &L.stepStart, start)) != NSF_OK) return st;
-      if ((st = dalloc(s, &L.stepPart, 9 * size_t(blocks))) != NSF_OK) return st;
-      const std::vector<unsigned long long> zero(1, 0ull);
-      if ((st = upload(s, &L.stepSync, zero)) != NSF_OK) return st;
-      L.stepShape = ch.shape;
-      L.stepPlanes = ch.planes;
-      L.stepSmem = smem;
-      L.stepBlocks = blocks;
+    }
+    StageItem* dItems = nullptr;
+    int* dStart = nullptr;
+    double* dPart = nullptr;
+    if ((st = upload(s, &dItems, items)) != NSF_OK) return st;
+    if ((st = upload(s, &dStart, start)) != NSF_OK) return st;
+    if ((st = dalloc(s, &dPart, parts)) != NSF_OK) return st;
+    const std::vector<unsigned long long> zero(STEP_WIDTHS, 0ull);
+    if ((st = upload(s, &L.stepSync, zero)) != NSF_OK) return st;
+    for (int w = 0; w < STEP_WIDTHS; ++w) {
+      L.step[w].items = dItems + itemsAt[w];
+      L.step[w].start = dStart + startAt[w];
+      L.step[w].part = dPart + partAt[w];
+      L.step[w].sync = L.stepSync + w;
     }
   }
   if (S.bodiesInteract && L.bcBlocks == 0) {  // the separate boundary kernels treat all bodies at once
@@ -703,7 +722,7 @@ nsf_status build_device(nsf_solver* s) {
   // one step as a CUDA graph
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   s->launchesPerStep = enqueue_step(s->dGrid, G, L, s->stream);
-  if (L.stepBlocks > 0) s->launchesPerStep = 1;
+  if (L.step[0].blocks > 0) s->launchesPerStep = 1;
   CK(cudaStreamEndCapture(s->stream, &s->graph));
   CK(cudaGraphInstantiate(&s->graphExec, s->graph, 0));
   return NSF_OK;
@@ -725,11 +744,72 @@ SnapInactive snap_inactive(const nsf_solver* s) {
 
 }  // namespace
 
+// A whole-step launch keeps its SMs until it ends, so handles that march at once would take turns on the GPU where their
+// launch sequences overlap. They run side by side instead: each takes a half of the SMs, or a quarter where there are
+// three or more, which costs a step little, since latency bounds it; grids above kSharedStepMaxNodes use the launch
+// sequence. Every path computes the same fields and dt bit for bit. Measured, us for a step of every handle, 1 / 2 / 4 / 8
+// handles, 16 steps queued at a time (every handle a launch sequence, before there was a whole-step kernel | whole-step
+// launches in turn | by this rule):
+//   sphere 32^3        119 127 147 219  |  58 116 232 463 |  58  68  84 168
+//   sphere 48^3        142 163 237 494  |  71 141 282 566 |  70 101 160 321
+//   Taylor-Green 64^3  111 187 306 653  | 102 204 408 817 | 101 173 294 622
+//   cylinder 161x83x3  218 328 558 1125 |  81 161 324 650 |  82 115 236 449
+// The line: half and quarter plans against launch sequences, 2 / 4 handles: 48^3 101 160 | 160 224, Taylor-Green 52^3
+// 125 232 | 135 240 (three handles 213 | 187), sphere 56^3 158 312 | 154 254.
+constexpr size_t kSharedStepMaxNodes = 120000;
+// Steps a launch, so that other streams' work gets its turn (1-3 ms); a launch costs 4-5 us, 0.3 us a step.
+constexpr uint64_t kStepsPerLaunch = 16;
+
+// Per device: the small-grid handles whose queued steps nobody has waited for yet, the most at once since there were
+// none, and the most of the time before that, which is what a handle that queues first has to go by. It decides how
+// much of the GPU a handle's coming steps take, never what they compute.
+struct Marching {
+  std::mutex m;
+  int now = 0, peak = 0, last = 0;
+};
+static Marching marchingOn[64];
+
+// Notes that steps are being queued; the handles to share the GPU with, this one included.
+static int steps_queued(nsf_solver* s) {
+  if (s->device >= 64) return 1;
+  Marching& d = marchingOn[s->device];
+  const std::lock_guard<std::mutex> lock(d.m);
+  if (!s->marching) {
+    s->marching = true;
+    d.peak = std::max(d.peak, ++d.now);
+  }
+  return std::max(d.peak, d.last);
+}
+static void steps_waited(nsf_solver* s) {
+  if (s->device < 0 || s->device >= 64) return;
+  Marching& d = marchingOn[s->device];
+  const std::lock_guard<std::mutex> lock(d.m);
+  if (!s->marching) return;
+  s->marching = false;
+  if (--d.now == 0) {
+    d.last = d.peak;
+    d.peak = 0;
+  }
+}
+
+// The plan for a handle's coming steps, or NULL for the launch sequence.
+static const StepPlan* step_plan(nsf_solver* s, bool wholeSteps) {
+  const StepPlan* p = s->plan.step;
+  if (p[0].blocks == 0) return nullptr;
+  const int handles = steps_queued(s);
+  if (handles <= 1) return &p[0];
+  if (s->setup.N > kSharedStepMaxNodes) return wholeSteps ? &p[0] : nullptr;
+  const StepPlan& q = p[handles == 2 ? 1 : 2];
+  return q.blocks > 0 ? &q : &p[0];
+}
+
 nsf_status nsf_queue_steps(nsf_solver* s, uint64_t nsteps, const StepTape& tape) {
-  if (s->plan.stepBlocks > 0) {
-    constexpr uint64_t perLaunch = 64;  // so that other streams' work gets its turn
-    for (uint64_t q = 0; q < nsteps; q += perLaunch)
-      CK(cudaError_t(launch_steps(s->hGrid, s->dGrid, s->plan, int(std::min(perLaunch, nsteps - q)), s->stream, tape)));
+  if (nsteps == 0) return NSF_OK;
+  const StepPlan* p = step_plan(s, tape.stage != nullptr);
+  if (p) {
+    for (uint64_t q = 0; q < nsteps; q += kStepsPerLaunch)
+      CK(cudaError_t(
+          launch_steps(s->hGrid, s->dGrid, s->plan, *p, int(std::min(kStepsPerLaunch, nsteps - q)), s->stream, tape)));
     return NSF_OK;
   }
   for (uint64_t q = 0; q < nsteps; ++q) CK(cudaGraphLaunch(s->graphExec, s->stream));
@@ -778,6 +858,7 @@ static nsf_status read_ctl(nsf_solver* s, StepCtl* out) {
   launch_ctl_out(s->dCtl, static_cast<StepCtl*>(dev), s->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s->stream));
+  steps_waited(s);
   *out = *s->hCtl;
   return NSF_OK;
 }
@@ -812,6 +893,7 @@ nsf_status nsf_download_planes(nsf_solver* s, uint32_t mask, size_t first, size_
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   cudaFree(tmp);
   if (e != cudaSuccess) return cuda_fail(s, e, "download");
+  steps_waited(s);
   return NSF_OK;
 }
 
@@ -1108,6 +1190,7 @@ nsf_status nsf_get_history(nsf_solver* s, uint64_t first, uint64_t count, double
   if (!s) return NSF_ERR_ARG;
   if (!s->initialized || s->hostOnly) return NSF_ERR_STATE;
   CK(cudaStreamSynchronize(s->stream));
+  steps_waited(s);
   StepCtl ctl;
   CK(cudaMemcpy(&ctl, s->dCtl, sizeof ctl, cudaMemcpyDeviceToHost));
   if (available) *available = ctl.level;
@@ -1133,6 +1216,7 @@ nsf_status nsf_march_timed(nsf_solver* s, uint64_t nsteps, double* elapsed_ms) {
   if (st != NSF_OK) return st;
   CK(cudaEventRecord(b, s->stream));
   CK(cudaEventSynchronize(b));
+  steps_waited(s);
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, a, b));
   cudaEventDestroy(a);
@@ -1204,6 +1288,7 @@ void nsf_destroy(nsf_solver* s) {
   if (s->stream) {
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
+    steps_waited(s);
   }
   if (s->graphExec) cudaGraphExecDestroy(s->graphExec);
   if (s->graph) cudaGraphDestroy(s->graph);

@@ -148,6 +148,19 @@ struct StageItem {
   int f0 = 0, f1 = 1 << 30;
 };
 
+// One plan of the whole-step kernel: `blocks` resident blocks run any number of steps in one launch.
+constexpr int STEP_WIDTHS = 3;
+struct StepPlan {
+  int blocks;
+  int shape;   // StepTile
+  int planes;  // most planes of a tile
+  size_t smem;
+  const StageItem* items;  // device; the tiles of block b are items[start[b] .. start[b + 1])
+  const int* start;
+  double* part;              // device, 9 x blocks end-of-step partials
+  unsigned long long* sync;  // device, grid barrier counter (a plan's own: it counts in multiples of blocks)
+};
+
 // Launch geometry of one step, fixed at initialisation.
 // Edge-condition kernels: blocks of 32 x kEdgeRows threads over a face (small blocks spread a face's
 // few thousand nodes over many SMs), listed one by one so that a launch holds only blocks with nodes
@@ -231,16 +244,10 @@ struct LaunchPlan {
   int* bcItems;
   int* bcItemStart;
   unsigned long long* bcSync;  // device, 1 + 2 members counters, zero at creation
-  // Whole-step kernel (nsf_step.cu) of a small single grid: stepBlocks resident blocks run any number of steps
-  // in one launch. 0: a step is the launch sequence above, captured as a graph.
-  int stepBlocks;
-  int stepShape;   // StepTile
-  int stepPlanes;  // most planes of a tile
-  size_t stepSmem;
-  StageItem* stepItems;  // device; the tiles of block b are stepItems[stepStart[b] .. stepStart[b + 1])
-  int* stepStart;
-  double* stepPart;               // device, 9 x stepBlocks end-of-step partials
-  unsigned long long* stepSync;   // device, grid barrier counter, zero at creation
+  // Whole-step kernel (nsf_step.cu) of a small single grid: its plans for all of the GPU's SMs, a half and a quarter of
+  // them. step[0].blocks == 0: a step is the launch sequence above, captured as a graph.
+  StepPlan step[STEP_WIDTHS];
+  unsigned long long* stepSync;  // device, the plans' barrier counters in order, zero at creation
   int nSlots;
   bool hasBodies;
   bool hasFilter, hasGhostWork, hasSolid;
@@ -271,7 +278,8 @@ struct StepTape {
   long long setWords = 0, perStage = 0;
   int nSets = 1;
 };
-int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream, const StepTape& tape = {});
+int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, const StepPlan& S, int nsteps, void* stream,
+                 const StepTape& tape = {});
 
 // Host entry points of nsf_kernels.cu.
 // Stage-kernel variant queries (v: StageTile).

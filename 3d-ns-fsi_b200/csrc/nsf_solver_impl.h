@@ -56,6 +56,7 @@ struct nsf_solver {
   struct AdjCtx* adj = nullptr;  // discrete-adjoint state (nsf_adjoint.cpp), created on first use
   // member of an ensemble or x-slab group: its steps are queued on the group's stream, not on `stream`
   bool grouped = false;
+  bool marching = false;  // steps of a small grid queued that nobody has waited for yet (counted per device, nsf_capi.cpp)
   // asynchronous downloads (nsf_download_async): a copy stream and two device staging buffers used in turn,
   // each with the events that mark its snapshot taken (on `stream`) and its copy to the host done (on
   // dlStream); ticket t uses buffer t & 1

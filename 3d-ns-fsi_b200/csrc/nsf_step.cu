@@ -478,7 +478,8 @@ int step_capacity(int shape, size_t smem, int nSM) {
   return std::min(nb, nb2) * nSM;
 }
 
-int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void* stream, const StepTape& tape) {
+int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, const StepPlan& S, int nsteps, void* stream,
+                 const StepTape& tape) {
   StepParams P{};
   P.bc.edges = L.bcEdges;
   P.bc.edgeStart = L.bcEdgeStart;
@@ -486,16 +487,16 @@ int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void
   P.bc.itemStart = L.bcItemStart;
   P.bc.levels = L.bcLevels;
   P.bc.members = 1;
-  P.items = L.stepItems;
-  P.start = L.stepStart;
-  P.part = L.stepPart;
-  P.sync = L.stepSync;
-  P.stashOffset = int(staged_bytes(L.stepShape, L.stepPlanes));
+  P.items = S.items;
+  P.start = S.start;
+  P.part = S.part;
+  P.sync = S.sync;
+  P.stashOffset = int(staged_bytes(S.shape, S.planes));
   P.tape = tape;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(L.stepBlocks));
+  cfg.gridDim = dim3(unsigned(S.blocks));
   cfg.blockDim = dim3(NT);
-  cfg.dynamicSmemBytes = L.stepSmem;
+  cfg.dynamicSmemBytes = S.smem;
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
@@ -503,7 +504,7 @@ int launch_steps(const Grid& hg, Grid* dg, const LaunchPlan& L, int nsteps, void
   cfg.attrs = at;
   cfg.numAttrs = 1;
   auto go = [&](auto kernel) { return int(cudaLaunchKernelEx(&cfg, kernel, hg, dg, P, nsteps)); };
-  if (L.stepShape == STEP_TILE_THIN) return tape.stage ? go(k_step<Thin, true>) : go(k_step<Thin, false>);
+  if (S.shape == STEP_TILE_THIN) return tape.stage ? go(k_step<Thin, true>) : go(k_step<Thin, false>);
   return tape.stage ? go(k_step<Cube, true>) : go(k_step<Cube, false>);
 }
 
