@@ -351,7 +351,8 @@ class Solver:
         return ms.value
 
     def profile_steps(self, nsteps):
-        """March nsteps launched eagerly; returns (mean ms of each stage kernel [4], mean ms per step)."""
+        """March nsteps (rounded up to tens) as replays of the launch sequence, also on a small grid, which march() does
+        not run by it; returns (mean ms of each stage kernel [4], mean ms per step)."""
         st = np.zeros(4)
         step = ctypes.c_double()
         self._check(lib().nsf_profile_steps(self.h, nsteps, _dp(st), ctypes.byref(step)))

@@ -7,7 +7,7 @@ A step is one RK4 step (Solver::marchTimeStep) over the whole grid. Each rank ru
 (the single-grid path does not shard), so value = ranks x nodes x K / max-over-ranks device time. The
 ensemble leg shards its members over the ranks (longest first, by node count) with no collective on the
 data path; its time is the slowest rank's.
-Timing: CUDA events on the solver's own stream around K graph-launched steps after W warm-up steps; the
+Timing: CUDA events on the solver's own stream around K queued steps after W warm-up steps; the
 resident fields (2.7 GB) are far larger than L2, so no flush is needed between steps.
 """
 import argparse
@@ -35,6 +35,7 @@ WORKLOADS = {
 }
 BYTES_PER_NODE_STEP = 680  # algorithmic HBM bytes per node per RK4 step (stage-fused scheme)
 STAGE_BYTES = [120, 200, 200, 160]
+STEPS_PER_LAUNCH = 16  # of a grid whose steps run in the whole-step kernel (launches_per_step() == 1; nsf_march)
 
 
 def measured_peak():
@@ -537,7 +538,7 @@ def main():
     import torch
     if dist:
         dist.barrier()
-    # The timed region (exactly K graph-launched steps between two events) is repeated R times; the line
+    # The timed region (exactly K queued steps between two events) is repeated R times; the line
     # reports the median, and the clock sampler runs across all repeats.
     reps_ms = []
     with ClockSampler(local) as clk:
@@ -553,17 +554,38 @@ def main():
     interior = int((cfg.NI - 2) * (cfg.NJ - 2) * (cfg.NK - 2))  # nodes whose RHS is computed
     launches = s.launches_per_step()
 
-    # dominant kernel: the four stage kernels timed by event nodes inside replays of a graph of consecutive
-    # steps (nsf_profile_steps), straight after the timed region; their share of those replays' step time,
-    # applied to the timed region's ms_per_step, is the stage kernels' time per step (it cannot exceed the
-    # step), and the roofline's achieved bandwidth follows from it
-    with ClockSampler(local) as clkp:
-        stage_ms, step_ms = s.profile_steps(max(args.steps, 50))
-    share = float(stage_ms.sum() / step_ms)
-    stage_step_ms = share * ms / args.steps
-    achieved = BYTES_PER_NODE_STEP * nodes / (stage_step_ms / 1e3) / 1e9
     peak, peak_kind = measured_peak()
-    traffic = profile_traffic(args.workload)
+    roof = {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None, "traffic": None,
+            "traffic_source": None, "algorithmic_bytes_per_node_step": BYTES_PER_NODE_STEP, "peak_kind": peak_kind,
+            # whole step (edge and control launches included): node-steps/s per GPU against
+            # the node-steps/s the peak bandwidth allows at 680 B per node-step
+            "step_frac": value / world / (peak * 1e9 / BYTES_PER_NODE_STEP)}
+    if launches == 1:
+        # a small grid: whole steps in one kernel, so its time per step is the timed region's
+        gpu_launches = -(-args.steps // STEPS_PER_LAUNCH)
+        stage_step_ms = ms / args.steps
+        roof["kernel"] = "k_step (one launch per %d steps; latency-bound, fields in L2)" % STEPS_PER_LAUNCH
+    else:
+        # dominant kernel: the four stage kernels timed by event nodes inside replays of a graph of consecutive
+        # steps (nsf_profile_steps), straight after the timed region; their share of those replays' step time,
+        # applied to the timed region's ms_per_step, is the stage kernels' time per step (it cannot exceed the
+        # step), and the roofline's achieved bandwidth follows from it
+        gpu_launches = launches * args.steps
+        with ClockSampler(local) as clkp:
+            stage_ms, step_ms = s.profile_steps(max(args.steps, 50))
+        share = float(stage_ms.sum() / step_ms)
+        stage_step_ms = share * ms / args.steps
+        # DRAM bytes per stage-kernel launch (mean of the four stages) from the committed ncu
+        # capture of this workload, next to the algorithmic bytes per launch
+        traffic = profile_traffic(args.workload)
+        if traffic:
+            roof["traffic"], roof["traffic_source"] = traffic["per_launch"], traffic["source"]
+        roof.update({"algorithmic_bytes_per_launch": BYTES_PER_NODE_STEP * nodes / 4,
+                     "kernel": "k_stage_ws (4 launches per step)", "stage_ms_per_step": round(stage_step_ms, 4),
+                     "stage_share": round(share, 4), "stage_ms_profiled": [round(x, 4) for x in stage_ms],
+                     "profile_step_ms": round(step_ms, 4), "profile_clocks": clkp.summary()})
+    roof["achieved"] = BYTES_PER_NODE_STEP * nodes / (stage_step_ms / 1e3) / 1e9
+    roof["frac"], roof["frac_of_8000"] = roof["achieved"] / peak, roof["achieved"] / 8000.0
     s.close()
 
     # end to end through the C ABI with host buffers: pinned upload of the initial state, K steps with
@@ -626,23 +648,10 @@ def main():
             "config": arm_config(args.workload, [int(cfg.NI), int(cfg.NJ), int(cfg.NK)], world),
             "e2e": e2e,
             "nonfinite": nonfinite[0],
-            "gpu_launches": launches * args.steps,
+            "gpu_launches": gpu_launches,
             "clocks": clk.summary(),
             "repeats": args.repeats, "ms_per_step_repeats": [round(x / args.steps, 5) for x in reps_ms],
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         # DRAM bytes per stage-kernel launch (mean of the four stages) from the committed ncu
-                         # capture of this workload, next to the algorithmic bytes per launch
-                         "traffic": traffic["per_launch"] if traffic else None,
-                         "traffic_source": traffic["source"] if traffic else None,
-                         "algorithmic_bytes_per_launch": BYTES_PER_NODE_STEP * nodes / 4,
-                         "kernel": "k_stage_ws (4 launches per step)", "stage_ms_per_step": round(stage_step_ms, 4),
-                         "stage_share": round(share, 4), "stage_ms_profiled": [round(x, 4) for x in stage_ms],
-                         "algorithmic_bytes_per_node_step": BYTES_PER_NODE_STEP, "peak_kind": peak_kind,
-                         "frac_of_8000": achieved / 8000.0, "profile_step_ms": round(step_ms, 4),
-                         # whole step (edge and control launches included): node-steps/s per GPU against
-                         # the node-steps/s the peak bandwidth allows at 680 B per node-step
-                         "step_frac": value / world / (peak * 1e9 / BYTES_PER_NODE_STEP),
-                         "profile_clocks": clkp.summary()},
+            "roofline": roof,
         }
         if snaps is not None:
             line["snapshots"] = snaps
