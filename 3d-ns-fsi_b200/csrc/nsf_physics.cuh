@@ -60,7 +60,8 @@ __device__ __forceinline__ double sqrt_nr(double a) {
 // Sutherland's viscosity x sqrt(x) sc1 / (re (T + sc1)), x = 1 + T, as x^2 / sqrt(x d^2) with d = re + T re/sc1 (C.muRe,
 // C.muA), with d's sign: one Newton-Raphson inverse square root in place of a square root and a reciprocal, twelve FP64
 // operations in place of twenty. The last iteration is written as a correction of r, which keeps its rounding out of the
-// result: rms error 1.21-1.29e-16 over |T| <= 0.2 (the quotient form: 1.31-1.35e-16), largest 5.6e-16 (5.7e-16).
+// result: measured against extended precision over |T| <= 0.2, rms error 1.25-1.33e-16 by the coefficients (the quotient
+// form: 1.28-1.50e-16), largest 5.4e-16 (6.6e-16); tests/test_viscosity_gpu.py.
 template <class CT>
 __device__ __forceinline__ double mu_nr(const CT& C, double x, double T) {
   const double d = fma(T, C.muA, C.muRe);
