@@ -1,5 +1,5 @@
 // C ABI implementation (include/nsfsi.h): the solver handle, device residency of all fields, the
-// device-side lists built from the host setup, and the queueing of steps: one cooperative launch for up to 16 steps of a
+// device-side lists built from the host setup, and the queueing of steps: one cooperative launch for up to 32 steps of a
 // small grid, one captured CUDA graph per RK4 step of the others.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -642,48 +642,36 @@ nsf_status build_device(nsf_solver* s) {
   if (!s->grouped && s->tileRequest < 0 && !std::getenv("NSF_STAGE_TILE") && L.bcBlocks > 0 && N <= kStepMaxNodes) {
     BcFlat fl;
     bc_flatten({&s->bcLevels}, fl);
-    std::vector<StageItem> items;  // the plans' lists, one after another
-    std::vector<int> start;
-    size_t itemsAt[STEP_WIDTHS] = {}, startAt[STEP_WIDTHS] = {}, partAt[STEP_WIDTHS] = {}, parts = 0;
+    const std::vector<unsigned long long> zero(STEP_WIDTHS, 0ull);
     for (int w = 0; w < STEP_WIDTHS; ++w) {
       StepPlan& p = L.step[w];
       const int nSM = std::max(1, s->nSM >> w);
       const StepChoice ch = step_choose(G.NI, G.NJ, G.NK, nSM);
       const StepShape t = step_shape(ch.shape);
       CK(cudaError_t(step_configure(ch.shape)));
-      p.shape = ch.shape;
-      p.planes = ch.planes;
-      p.smem = step_smem_bytes(ch.shape, ch.planes, L.bcLevels);
+      const size_t smem = step_smem_bytes(ch.shape, ch.planes, L.bcLevels);
       const int warps = int(std::min<long long>((fl.maxWork + 31) / 32, nSM));
-      p.blocks = std::min(std::max(ch.items, warps), step_capacity(ch.shape, p.smem, nSM));
-      itemsAt[w] = items.size();
-      startAt[w] = start.size();
-      partAt[w] = parts;
-      parts += 9 * size_t(std::max(0, p.blocks));
-      std::vector<StageItem> all;
+      const int blocks = std::min(std::max(ch.items, warps), step_capacity(ch.shape, smem, nSM));
+      if (blocks <= 0) break;
+      std::vector<StageItem> all, ordered;
       for (int c0 = 1; c0 <= planes; c0 += ch.planes)
         for (int j0 = 1; j0 <= G.NJ - 2; j0 += t.tj)
           for (int k0 = 1; k0 <= G.NK - 2; k0 += t.tk)
             all.push_back(StageItem{j0, k0, c0, std::min(planes, c0 + ch.planes - 1), 0});
-      start.push_back(0);
-      for (int b = 0; b < p.blocks; ++b) {
-        for (size_t q = size_t(b); q < all.size(); q += size_t(p.blocks)) items.push_back(all[q]);
-        start.push_back(int(items.size() - itemsAt[w]));
+      std::vector<int> start(1, 0);
+      for (int b = 0; b < blocks; ++b) {
+        for (size_t q = size_t(b); q < all.size(); q += size_t(blocks)) ordered.push_back(all[q]);
+        start.push_back(int(ordered.size()));
       }
-    }
-    StageItem* dItems = nullptr;
-    int* dStart = nullptr;
-    double* dPart = nullptr;
-    if ((st = upload(s, &dItems, items)) != NSF_OK) return st;
-    if ((st = upload(s, &dStart, start)) != NSF_OK) return st;
-    if ((st = dalloc(s, &dPart, parts)) != NSF_OK) return st;
-    const std::vector<unsigned long long> zero(STEP_WIDTHS, 0ull);
-    if ((st = upload(s, &L.stepSync, zero)) != NSF_OK) return st;
-    for (int w = 0; w < STEP_WIDTHS; ++w) {
-      L.step[w].items = dItems + itemsAt[w];
-      L.step[w].start = dStart + startAt[w];
-      L.step[w].part = dPart + partAt[w];
-      L.step[w].sync = L.stepSync + w;
+      if ((st = upload(s, &p.items, ordered)) != NSF_OK) return st;
+      if ((st = upload(s, &p.start, start)) != NSF_OK) return st;
+      if ((st = dalloc(s, &p.part, 9 * size_t(blocks))) != NSF_OK) return st;
+      if (w == 0 && (st = upload(s, &L.stepSync, zero)) != NSF_OK) return st;
+      p.sync = L.stepSync + w;
+      p.shape = ch.shape;
+      p.planes = ch.planes;
+      p.smem = smem;
+      p.blocks = blocks;
     }
   }
   if (S.bodiesInteract && L.bcBlocks == 0) {  // the separate boundary kernels treat all bodies at once
@@ -757,8 +745,8 @@ SnapInactive snap_inactive(const nsf_solver* s) {
 // The line: half and quarter plans against launch sequences, 2 / 4 handles: 48^3 101 160 | 160 224, Taylor-Green 52^3
 // 125 232 | 135 240 (three handles 213 | 187), sphere 56^3 158 312 | 154 254.
 constexpr size_t kSharedStepMaxNodes = 120000;
-// Steps a launch, so that other streams' work gets its turn (1-3 ms); a launch costs 4-5 us, 0.3 us a step.
-constexpr uint64_t kStepsPerLaunch = 16;
+// Steps a launch, so that other streams' work gets its turn (after 2-6 ms); a launch costs 4-7 us, 0.2 us a step.
+constexpr uint64_t kStepsPerLaunch = 32;
 
 // Per device: the small-grid handles whose queued steps nobody has waited for yet, the most at once since there were
 // none, and the most of the time before that, which is what a handle that queues first has to go by. It decides how

@@ -155,8 +155,8 @@ struct StepPlan {
   int shape;   // StepTile
   int planes;  // most planes of a tile
   size_t smem;
-  const StageItem* items;  // device; the tiles of block b are items[start[b] .. start[b + 1])
-  const int* start;
+  StageItem* items;  // device; the tiles of block b are items[start[b] .. start[b + 1])
+  int* start;
   double* part;              // device, 9 x blocks end-of-step partials
   unsigned long long* sync;  // device, grid barrier counter (a plan's own: it counts in multiples of blocks)
 };

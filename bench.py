@@ -35,7 +35,7 @@ WORKLOADS = {
 }
 BYTES_PER_NODE_STEP = 680  # algorithmic HBM bytes per node per RK4 step (stage-fused scheme)
 STAGE_BYTES = [120, 200, 200, 160]
-STEPS_PER_LAUNCH = 16  # of a grid whose steps run in the whole-step kernel (launches_per_step() == 1; nsf_march)
+STEPS_PER_LAUNCH = 32  # of a grid whose steps run in the whole-step kernel (launches_per_step() == 1; nsf_march)
 
 
 def measured_peak():

@@ -113,7 +113,7 @@ nsf_status nsf_initialize(nsf_solver* s);
 
 /* Replaces `nsteps` calls of Solver::marchTimeStep(t, timeLevel) (Solver.cpp:130-167). Asynchronous:
  * the steps are queued on the handle's stream (one CUDA graph per step; for small grids launches of
- * up to 16 steps each, which share the GPU's SMs with other small handles whose steps are in flight). In end_time mode, steps after
+ * up to 32 steps each, which share the GPU's SMs with other small handles whose steps are in flight). In end_time mode, steps after
  * t reaches t_end are no-ops, as Simulation::run (Simulation.cpp:19-30) would not call them. */
 nsf_status nsf_march(nsf_solver* s, uint64_t nsteps);
 

@@ -10,7 +10,7 @@ import bench
 from test_bench_cpu import STEP_MS, fake_nsfsi
 
 
-@pytest.mark.parametrize("steps,launches", [(1, 1), (16, 1), (17, 2), (200, 13)])
+@pytest.mark.parametrize("steps,launches", [(1, 1), (32, 1), (33, 2), (200, 7)])
 def test_small_grid_line_describes_the_kernel_that_ran(steps, launches, monkeypatch, capsys):
     m = fake_nsfsi()
 
