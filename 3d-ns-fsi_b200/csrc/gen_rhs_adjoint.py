@@ -13,7 +13,7 @@ with the reference's stencil coefficients. From it this script emits
     the tests as an independent check of the emitted code and of the term table against the oracle.
 
 The adjoint kernel evaluates the same transposed stencil in flux form (nsf_rhs_adjoint_flux.cuh, about a quarter of the
-operations); the tests compare it with the numpy gather here.
+operations); the tests compare it with the numpy gather here, and the emitted gather, which no kernel uses any more, too.
 
     python 3d-ns-fsi_b200/csrc/gen_rhs_adjoint.py      (rewrites nsf_rhs_adjoint.cuh)
 """

@@ -637,7 +637,7 @@ nsf_status build_device(nsf_solver* s) {
   }
   // Small grids: the whole-step kernel (its boundary work needs the fused plan above). The line lies where a step
   // of the launch sequence costs as much (us per step, graph / whole-step kernel, one B200): Taylor-Green 64^3
-  // 104 / 100, 80^3 177 / 167, 84^3 193 / 228; channel with a sphere 64^3 142 / 118, 80^3 226 / 190, 88^3 263 / 269.
+  // 106 / 102, 80^3 180 / 168, 84^3 198 / 228; channel with a sphere 64^3 142 / 117, 80^3 215 / 189, 88^3 250 / 269.
   // A requested tile shape (ensemble members, the tuner, NSF_STAGE_TILE) means the streaming stage kernel.
   if (!s->grouped && s->tileRequest < 0 && !std::getenv("NSF_STAGE_TILE") && L.bcBlocks > 0 && N <= kStepMaxNodes) {
     BcFlat fl;

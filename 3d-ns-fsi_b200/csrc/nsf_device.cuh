@@ -30,6 +30,8 @@ struct Consts {
   double muRe, muA;  // re and re / sc1, kept where mu_nr can square them
   // continuity / inviscid: -1/(2d)
   double ax, ay, az;
+  // (The kernels read the energy's coefficients e_* for the momenta too, which have the same values; the momenta's own,
+  // xm_* to zm_*, are those the term table of gen_rhs_adjoint.py names.)
   // x-momentum: 2/(3dx^2), 1/(2dy^2), 1/(2dz^2), -1/(6dydx), 1/(4dxdy), -1/(6dzdx), 1/(4dxdz)
   double xm_xx, xm_yy, xm_zz, xm_yx, xm_xy, xm_zx, xm_xz;
   // y-momentum: 1/(2dx^2), 2/(3dy^2), 1/(2dz^2), -1/(6dxdy), 1/(4dydx), -1/(6dzdy), 1/(4dydz)
@@ -87,9 +89,9 @@ struct Grid {
   double* bufs[3][5];
   double* acc[5];
   int NKp;                // k pitch of the device layout (multiple of 4: rows start on 32-byte boundaries)
-  const void* tmaps;      // device array of TMA descriptors (see nsf_stage_tma.cu)
+  const void* tmaps;      // device array of TMA descriptors (see nsf_stage_ws.cu)
   const uint8_t* type;    // NodeTypeEnum | FILTER_BIT | EDGE_PLANE_BIT | ZCOPY_UP_BIT | ZCOPY_DOWN_BIT
-  const int* fidx;        // node -> filter slot (only read where FILTER_BIT is set)
+  const int* fidx;        // node -> its first filter slot, -1 where FILTER_BIT is not set (NULL without filter nodes)
   double* fpre;           // [F][2] pre-filter rho, rho_E of the last near-body filter
   double* fnew;           // [F][2] filtered values (written back after the ghost update)
   const uint8_t* fsolid;  // [F] bit q: stencil node q (centre, +i, -i, +j, -j, +k, -k) is a solid node off the faces

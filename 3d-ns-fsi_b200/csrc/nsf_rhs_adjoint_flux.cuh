@@ -10,7 +10,8 @@
 //   the differences D_b u_c of its neighbours, which read this node's velocities: S_bc(X - b) - S_bc(X + b) with S_bc
 //   the adjoint of D_b u_c at a node (mixed_adjoint).
 // Each product is formed once per node or face, about 500 FP64 operations a node, where the term-by-term gather over
-// the 19 RHS nodes that read a node (nsf_rhs_adjoint.cuh, the form the tests compare this one with) takes 2,000.
+// the 19 RHS nodes that read a node takes 2,000 (nsf_rhs_adjoint.cuh, which no kernel uses any more: the tests evaluate
+// it against the term table of gen_rhs_adjoint.py, and this form against the same table).
 //
 // lam(e, di, dj, dk): RHS adjoint of equation e at offset (di, dj, dk), zero where no RHS is taken. val(q, di, dj, dk):
 // u, v, w, T, mu for q = 0..4. kappa = pf mu is not an input of its own: its adjoint is part of mu's.

@@ -17,8 +17,8 @@
 //     see x_node / x_face in nsf_physics.cuh) and carries them in registers along the column; the
 //     RHS of the previous plane is then G/F differences plus the y/z terms read from the staged planes,
 //     and the RK4 combine is written with coalesced 256-byte row stores.
-// Warpgroup 0 runs with 88 registers per thread and the column warpgroups with 208 (setmaxnreg; 104 and 200 with
-// filter nodes), so the register-hungry RHS does not spill while the CTA still has twelve warps.
+// Warpgroup 0 runs with 104 registers per thread and the column warpgroups with 200 (setmaxnreg; 88 and 208 in an
+// ensemble's stage 4), so the register-hungry RHS does not spill while the CTA still has twelve warps.
 //
 // Ring slots have a "full" and an "empty" mbarrier. Every wait is bounded: a wait that gives up sets
 // StepCtl::timeout and a CTA-wide abort flag that ends every other wait at once; the producer then

@@ -18,8 +18,9 @@
 // in the launch are read through L2 (__ldcg). Arithmetic and its order per node are the streaming kernel's and
 // k_bc's, so the fields equal theirs bit for bit (ensembles, x-slabs and the adjoint use those kernels).
 //
-// Measured (us per step, before as a graph of ten launches / now, one B200): sphere 32^3 117 / 57, sphere 48^3
-// 147 / 72, cylinder 161x83x3 217 / 82, walls and two spheres 75x53x61 193 / 131, Taylor-Green 64^3 110 / 101.
+// Measured (us per step: by the launch sequence / by this kernel, one B200): sphere 32^3 101 / 57, sphere 48^3 123 / 71,
+// cylinder 161x83x3 188 / 82, walls and a sphere 75x53x61 158 / 131, Taylor-Green 64^3 106 / 102 (the launch sequence
+// as it was before this kernel came: 119, 142, 218, 186, 111).
 // A step of sphere 48^3 (SM cycles of a block at 1.9 GHz, 141 K in all): four stage phases of 13-15 K (4.3 K the
 // staged planes, 9.5 K the RHS: two planes a thread, half of the FP64 rate), four boundary phases of 3-5 K edges
 // and 4-6 K ghosts, a barrier about 2.2 K from the last arrival to the release (memory latency), 8 K the end and
@@ -47,7 +48,7 @@ constexpr int NG = NT / NCOL;  // groups of threads that share a tile's planes
 constexpr int NQ = 9;          // end-of-step quantities: four dt maxima, five change-norm sums
 constexpr int kStash = 3;      // boundary levels whose first item per thread is kept in shared memory
 constexpr int kTileStash = 16;
-constexpr size_t kSmemBudget = 200 * 1024;  // staged planes of a tile
+constexpr size_t kSmemBudget = 200 * 1024;  // staged planes of a tile (227 KB a block less the stash and the copies)
 
 struct StepParams {
   BcParams bc;
@@ -434,7 +435,11 @@ size_t step_smem_bytes(int shape, int planes, int levels) {
 
 // The tile shape, the planes per tile and the blocks that run them: the smallest estimated time of one stage. A
 // block's tile costs a fixed part (load latency, barriers), one pass of the block over the tile's halo nodes
-// per NT of them, and one pass over its planes per NG of them plus the start of the carried x quantities.
+// per NT of them, and one pass over its planes per NG of them plus the start of the carried x quantities. The weights
+// are relative; the choice they make was the fastest of 1 .. 12 planes on each grid measured (us per step at 2 .. 10
+// planes by the plane): sphere 48^3 (6 chosen) 85 78 87 93 71 78 81 84 89, walls 75x53x61 (8) 154 146 144 132 138 143 131
+// 139 148, Taylor-Green 64^3 (7) 132 121 120 108 115 102 106 112 122, 80^3 (10) 233 195 186 183 170 182 178 179 168;
+// sphere 32^3 2 planes, cylinder 161x83x3 4.
 StepChoice step_choose(int NI, int NJ, int NK, int nSM) {
   StepChoice best{};
   double bestCost = 1e300;
