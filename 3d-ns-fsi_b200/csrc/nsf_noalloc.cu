@@ -20,7 +20,10 @@
 // What bounds it: HBM, 80 bytes a node (two states of five fields, read once). The first pass runs a fixed number of
 // blocks, whose threads stride over the nodes with their sums and maxima in registers, so that the nine block
 // reductions come once per block instead of once per 256 nodes and the final pass reads a few thousand partials, not
-// one per 256 nodes. Measured at 192^3 (566 MB): 231 us (170 + 69 us of kernels) before, 103 us now (5.5 TB/s).
+// one per 256 nodes. Measured at 192^3 (566 MB): 231 us (170 + 69 us of kernels) before, 105 us now (5.4 TB/s). Quotients
+// are corrected by their residuals and a block's warps are added in pairs, so that dt and norms are no further from an
+// evaluation in 64 bits than by divisions and one partial per 256 nodes (rms over 40 states: 192^3 6.6e-17, 6.8e-17
+// before; 8.8e-17 with plain products and the warps one after another, which took 2 us less).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -67,10 +70,13 @@ __device__ __forceinline__ double block_reduce(const double (&v)[kQ], double (&r
     if (lane == 0) red[q][wid] = a;
   }
   __syncthreads();
+  static_assert(kThreads == 256, "eight warps, in pairs");
   double a = 0;
   if (threadIdx.x < kQ) {
-    a = red[threadIdx.x][0];
-    for (int w = 1; w < kThreads / 32; ++w) a = combine(threadIdx.x, a, red[threadIdx.x][w]);
+    const int q = threadIdx.x;
+    const double* w = red[q];
+    a = combine(q, combine(q, combine(q, w[0], w[1]), combine(q, w[2], w[3])),
+                combine(q, combine(q, w[4], w[5]), combine(q, w[6], w[7])));
   }
   return a;
 }
@@ -98,17 +104,18 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
       const double d = o[f] - u[f];
       v[f] += interior ? d * d : 0.0;
     }
-    const double r1 = nsf::recip_nr(u[0] + 1.0);
+    const double a1 = u[0] + 1.0, r1 = nsf::recip_nr(a1);
     const double uu = u[1] * r1, vv = u[2] * r1, ww = u[3] * r1;
     const double pp = p.gm1 * (u[4] - (u[0] + 1.0) * 0.5 * (uu * uu + vv * vv + ww * ww));
     const double T = (p.gamma * pp - u[0]) * r1;
     const double x = 1.0 + T;
-    const double mu = x * nsf::sqrt_nr(x) * p.sc1 * nsf::recip_nr(p.re * (T + p.sc1));
-    const double c = nsf::sqrt_nr((1.0 + p.gamma * pp) * r1);
+    const double den = p.re * (T + p.sc1);
+    const double mu = nsf::quot_nr(x * nsf::sqrt_nr(x) * p.sc1, den, nsf::recip_nr(den));
+    const double c = nsf::sqrt_nr(nsf::quot_nr(1.0 + p.gamma * pp, a1, r1));
     v[5] = fmax(v[5], c + fabs(uu));
     v[6] = fmax(v[6], c + fabs(vv));
     v[7] = fmax(v[7], c + fabs(ww));
-    v[8] = fmax(v[8], mu * r1 * p.vmod);
+    v[8] = fmax(v[8], nsf::quot_nr(mu, a1, r1) * p.vmod);
     k += p.sK;
     j += p.sJ;
     i += p.sI;

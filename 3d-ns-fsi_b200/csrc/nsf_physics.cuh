@@ -57,6 +57,13 @@ __device__ __forceinline__ double sqrt_nr(double a) {
   return fma(fma(-s, s, a), 0.5 * r, s);
 }
 
+// a / b from b's refined reciprocal r, corrected by the quotient's residual: rounded as the division but for rare cases
+// next to a midpoint, where the product a r is off by one in the last place every few values.
+__device__ __forceinline__ double quot_nr(double a, double b, double r) {
+  const double q = a * r;
+  return fma(r, fma(-b, q, a), q);
+}
+
 // Sutherland's viscosity x sqrt(x) sc1 / (re (T + sc1)), x = 1 + T, as x^2 / sqrt(x d^2) with d = re + T re/sc1 (C.muRe,
 // C.muA), with d's sign: one Newton-Raphson inverse square root in place of a square root and a reciprocal, twelve FP64
 // operations in place of twenty. The last iteration is written as a correction of r, which keeps its rounding out of the
