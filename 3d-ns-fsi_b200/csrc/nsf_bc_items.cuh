@@ -167,7 +167,7 @@ __device__ __forceinline__ void edge_node(const Grid& G, const StepCtl* c, const
           if (primKnown)
             dt_terms_known(C, cv[0], u, v, w, p, T, dta);
           else
-            dt_terms(C, cv, dta);
+            dt_terms_bc(C, cv, dta);
           for (int f = 0; f < 5; ++f) bad |= !isfinite(cv[f]);
         }
       }
@@ -264,7 +264,7 @@ __device__ __forceinline__ void ghost_node(const Grid& G, const StepCtl* c, int 
   const double gc[5] = {ip[0], -ip[1], -ip[2], -ip[3], ip[4]};
   for (int f = 0; f < 5; ++f) O[f][n] = gc[f];
   if (s == 3 && G.glast[q]) {  // a node in two bodies' ghost lists: the dt terms of its final values
-    dt_terms(G.C, gc, dta);
+    dt_terms_bc(G.C, gc, dta);
     for (int f = 0; f < 5; ++f) bad |= !isfinite(gc[f]);
   }
 }
@@ -281,7 +281,7 @@ __device__ __forceinline__ void inactive_node(const Grid& G, const StepCtl* c, i
   if (isnan(pr[0])) {  // periodic copy of a node whose primitives follow its conserved values
     const double v[5] = {r0, ld_res(c, s, 1, n, true), ld_res(c, s, 2, n, true), ld_res(c, s, 3, n, true),
                          ld_res(c, s, 4, n, true)};
-    dt_terms(G.C, v, dta);
+    dt_terms_bc(G.C, v, dta);
   } else {
     dta.add(G.C, r0, pr[0], pr[1], pr[2], pr[3], pr[4]);
   }

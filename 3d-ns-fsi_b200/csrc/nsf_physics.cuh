@@ -129,25 +129,41 @@ struct DtAcc {
 // dt-limit terms of a node (getInviscidTimeStepLimit / getViscousTimeStepLimit, Solver.cpp:91-126) with one
 // reciprocal of 1 + rho for all the divisions by it, reciprocals and square roots by Newton-Raphson (recip_nr,
 // sqrt_nr). The terms only enter maxima, so their last-bit rounding moves dt by at most an ulp or two.
-// dt_terms_at: velocities, pressure and temperature known, r1 = 1 / (1 + rho).
-__device__ __forceinline__ void dt_terms_at(const Consts& C, double r1, double u, double v, double w, double p, double T,
-                                            DtAcc& a) {
-  const double c = sqrt_nr((1.0 + C.gamma * p) * r1);
-  a.sx = fmax(a.sx, c + fabs(u));
-  a.sy = fmax(a.sy, c + fabs(v));
-  a.sz = fmax(a.sz, c + fabs(w));
-  a.nu = fmax(a.nu, mu_nr(C, 1.0 + T, T) * r1 * C.vmod);
-}
+// dt_terms: the stage kernels' interior nodes. dt_terms_bc: edge, ghost and inactive nodes, whose quotients are
+// corrected by their residuals (the rounding of the divisions); dt_terms_known: the same with velocities, pressure and
+// temperature known.
 __device__ __forceinline__ void dt_terms(const Consts& C, const double (&u)[5], DtAcc& a) {
   const double r1 = recip_nr(u[0] + 1.0);
   const double vx = u[1] * r1, vy = u[2] * r1, vz = u[3] * r1;
   const double p = C.gm1 * (u[4] - 0.5 * (u[1] * vx + u[2] * vy + u[3] * vz));
   const double T = (C.gamma * p - u[0]) * r1;
-  dt_terms_at(C, r1, vx, vy, vz, p, T, a);
+  const double c = sqrt_nr((1.0 + C.gamma * p) * r1);
+  a.sx = fmax(a.sx, c + fabs(vx));
+  a.sy = fmax(a.sy, c + fabs(vy));
+  a.sz = fmax(a.sz, c + fabs(vz));
+  a.nu = fmax(a.nu, mu_nr(C, 1.0 + T, T) * r1 * C.vmod);
+}
+__device__ __forceinline__ void dt_terms_at(const Consts& C, double r, double r1, double u, double v, double w, double p,
+                                            double T, DtAcc& a) {
+  const double c = sqrt_nr(quot_nr(1.0 + C.gamma * p, r, r1));
+  const double x = 1.0 + T, den = C.re * (T + C.sc1);
+  const double mu = quot_nr(x * sqrt_nr(x) * C.sc1, den, recip_nr(den));
+  a.sx = fmax(a.sx, c + fabs(u));
+  a.sy = fmax(a.sy, c + fabs(v));
+  a.sz = fmax(a.sz, c + fabs(w));
+  a.nu = fmax(a.nu, quot_nr(mu, r, r1) * C.vmod);
+}
+__device__ __forceinline__ void dt_terms_bc(const Consts& C, const double (&u)[5], DtAcc& a) {
+  const double r = u[0] + 1.0, r1 = recip_nr(r);
+  const double vx = u[1] * r1, vy = u[2] * r1, vz = u[3] * r1;
+  const double p = C.gm1 * (u[4] - r * 0.5 * (vx * vx + vy * vy + vz * vz));
+  const double T = (C.gamma * p - u[0]) * r1;
+  dt_terms_at(C, r, r1, vx, vy, vz, p, T, a);
 }
 __device__ __forceinline__ void dt_terms_known(const Consts& C, double rho, double u, double v, double w, double p,
                                                double T, DtAcc& a) {
-  dt_terms_at(C, recip_nr(rho + 1.0), u, v, w, p, T, a);
+  const double r = rho + 1.0;
+  dt_terms_at(C, r, recip_nr(r), u, v, w, p, T, a);
 }
 
 __device__ __forceinline__ double warp_max(double v) {
