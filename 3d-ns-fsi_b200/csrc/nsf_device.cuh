@@ -133,7 +133,8 @@ struct Grid {
   StepCtl* ctlHist;         // [nCtlHist]: the control block of step n right after its prologue (roles)
   int nCtlHist;
   // reductions
-  double* normPart;         // [nNormSlots][5]: stage-kernel CTAs first, then the near-body filter's blocks
+  double* normPart;         // [nNormSlots][5]: the stage kernel's CTAs (an ensemble member: its items' column warps) first,
+                            // then the near-body filter's blocks
   int nNormSlots;
   int normSlotFilter;       // first slot of the near-body filter's partial sums
   double* hist;             // [MAX_HIST][7]
@@ -148,7 +149,9 @@ struct StageItem {
   // staged planes that may hold near-body filter nodes within the tile and its halo, inclusive (mark_filter_planes;
   // the default is every plane)
   int f0 = 0, f1 = 1 << 30;
+  int slot = 0;  // ensembles: the first of the item's stageNormSlots change-norm slots among its member's
 };
+constexpr int stageNormSlots = 8;  // one per column warp of a stage CTA
 
 // One plan of the whole-step kernel: `blocks` resident blocks run any number of steps in one launch.
 constexpr int STEP_WIDTHS = 3;

@@ -130,6 +130,8 @@ nsf_status build_members_plan(const std::vector<nsf_solver*>& members, int nSM, 
   L.stageSpan = int(best);
   for (int g = 0; g < M; ++g)
     mark_filter_planes(members[g]->hGrid, members[g]->filterNodes, TJ, TK, g, ordered);
+  std::vector<int> itemsOf(size_t(M), 0);
+  for (StageItem& w : ordered) w.slot = stageNormSlots * itemsOf[size_t(w.g)]++;
   L.nItems = int(ordered.size());
   L.stageBlocks = int(start.size()) - 1;
   nsf_status st;
@@ -195,18 +197,18 @@ nsf_status build_members_plan(const std::vector<nsf_solver*>& members, int nSM, 
       CKP(cudaMemset(L.bcSync, 0, (2 * size_t(M) + 1) * sizeof(unsigned long long)));
     }
   }
-  // member grids: the stage kernel adds its norm partials into slot 0 of each member, the near-body
-  // filter's blocks (or the fused boundary kernel's) use slots 1 .. filterBlocks
+  // member grids: the stage kernel writes its norm partials into the member's first slots, stageNormSlots an item, the
+  // near-body filter's blocks (or the fused boundary kernel's) use the filterBlocks after them
   hGrids.resize(M);
   for (int g = 0; g < M; ++g) {
     Grid G = members[g]->hGrid;
-    const int slots = 1 + L.filterBlocks;
+    const int slots = stageNormSlots * itemsOf[size_t(g)] + L.filterBlocks;
     double* norm = nullptr;
     if ((st = group_alloc(allocs, err, &norm, 5 * size_t(slots))) != NSF_OK) return st;
     CKP(cudaMemset(norm, 0, 5 * size_t(slots) * sizeof(double)));
     G.normPart = norm;
     G.nNormSlots = slots;
-    G.normSlotFilter = 1;
+    G.normSlotFilter = stageNormSlots * itemsOf[size_t(g)];
     hGrids[g] = G;
   }
   if ((st = group_alloc(allocs, err, dGrids, size_t(M))) != NSF_OK) return st;

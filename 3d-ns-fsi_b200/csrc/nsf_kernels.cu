@@ -32,7 +32,6 @@ namespace nsf {
 // Start of a step (prologue_warp). Member m = blockIdx.x of the grid array (a single grid: one block).
 __global__ void k_prologue(Grid* grids) {
   const Grid& G = grids[blockIdx.x];
-  if (threadIdx.x < 5) G.normPart[threadIdx.x] = 0.0;  // slot 0: the ensemble stage kernel adds into it
   prologue_warp(G, G.ctl, threadIdx.x, true);
 }
 

@@ -27,8 +27,7 @@
 // The node values and the dt sequence equal the single-grid solve's bit for bit:
 // every node's dt terms are formed by the same kernel as in the whole grid (the periodic x faces' by their
 // edge items, BC_SLAB_COPY), and maxima do not depend on the order; the change norms are summed slab by slab,
-// so they agree to rounding (also from run to run: a stage launch over several slabs adds them with
-// atomics, as an ensemble's does). Immersed bodies are not supported across slabs (NSF_ERR_ARG).
+// so they agree to rounding. Immersed bodies are not supported across slabs (NSF_ERR_ARG).
 #include <cuda_runtime.h>
 
 #include <algorithm>
