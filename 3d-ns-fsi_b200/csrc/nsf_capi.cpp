@@ -748,25 +748,40 @@ constexpr size_t kSharedStepMaxNodes = 120000;
 // Steps a launch, so that other streams' work gets its turn (after 2-6 ms); a launch costs 4-7 us, 0.2 us a step.
 constexpr uint64_t kStepsPerLaunch = 32;
 
+// Beside steps of a large grid, an ensemble or a slab group small grids use the launch sequence, too: a whole-step launch
+// would keep the others' kernels, which take all SMs for a fraction of a step, waiting for many steps of the small one
+// (sphere 32^3, 400 steps, beside Taylor-Green 128^3, 50 steps, ms until both / the large one are done: whole-step
+// launches 44 / 44, by this rule 58 / 23, before there was a whole-step kernel 66 / 24).
+
 // Per device: the small-grid handles whose queued steps nobody has waited for yet, the most at once since there were
-// none, and the most of the time before that, which is what a handle that queues first has to go by. It decides how
-// much of the GPU a handle's coming steps take, never what they compute.
+// none, and the most of the time before that, which is what a handle that queues first has to go by; the other handles
+// and groups with steps in flight, and whether there were any beside small ones since, and the time before. It decides
+// how a handle's coming steps are launched, never what they compute.
 struct Marching {
   std::mutex m;
   int now = 0, peak = 0, last = 0;
+  int large = 0;
+  bool beside = false, besideLast = false;
 };
 static Marching marchingOn[64];
 
-// Notes that steps are being queued; the handles to share the GPU with, this one included.
+static bool whole_steps(const nsf_solver* s) { return s->plan.step[0].blocks > 0; }
+
+// Notes that steps of s are being queued. The small handles to share the GPU with, this one included; 0: there are
+// large ones beside them.
 static int steps_queued(nsf_solver* s) {
-  if (s->device >= 64) return 1;
+  if (s->device < 0 || s->device >= 64) return 1;
   Marching& d = marchingOn[s->device];
   const std::lock_guard<std::mutex> lock(d.m);
   if (!s->marching) {
     s->marching = true;
-    d.peak = std::max(d.peak, ++d.now);
+    if (whole_steps(s))
+      d.peak = std::max(d.peak, ++d.now);
+    else
+      ++d.large;
   }
-  return std::max(d.peak, d.last);
+  if (d.now > 0 && d.large > 0) d.beside = true;
+  return d.beside || d.besideLast ? 0 : std::max(d.peak, d.last);
 }
 static void steps_waited(nsf_solver* s) {
   if (s->device < 0 || s->device >= 64) return;
@@ -774,19 +789,25 @@ static void steps_waited(nsf_solver* s) {
   const std::lock_guard<std::mutex> lock(d.m);
   if (!s->marching) return;
   s->marching = false;
-  if (--d.now == 0) {
+  if (!whole_steps(s)) {
+    --d.large;
+  } else if (--d.now == 0) {
     d.last = d.peak;
     d.peak = 0;
+    d.besideLast = d.beside;
+    d.beside = false;
   }
 }
+void nsf_steps_queued(nsf_solver* s) { steps_queued(s); }
+void nsf_steps_waited(nsf_solver* s) { steps_waited(s); }
 
 // The plan for a handle's coming steps, or NULL for the launch sequence.
 static const StepPlan* step_plan(nsf_solver* s, bool wholeSteps) {
   const StepPlan* p = s->plan.step;
-  if (p[0].blocks == 0) return nullptr;
   const int handles = steps_queued(s);
-  if (handles <= 1) return &p[0];
-  if (s->setup.N > kSharedStepMaxNodes) return wholeSteps ? &p[0] : nullptr;
+  if (!whole_steps(s)) return nullptr;
+  if (handles == 1) return &p[0];
+  if (handles == 0 || s->setup.N > kSharedStepMaxNodes) return wholeSteps ? &p[0] : nullptr;
   const StepPlan& q = p[handles == 2 ? 1 : 2];
   return q.blocks > 0 ? &q : &p[0];
 }

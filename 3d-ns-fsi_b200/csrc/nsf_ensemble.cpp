@@ -446,6 +446,7 @@ nsf_status nsf_ensemble_march(nsf_ensemble* e, uint64_t nsteps) {
   if (!e) return NSF_ERR_ARG;
   if (!e->graphExec) return NSF_ERR_STATE;
   CKE(cudaSetDevice(e->device));
+  if (nsteps) nsf_steps_queued(e->members[0]);
   for (uint64_t q = 0; q < nsteps; ++q) CKE(cudaGraphLaunch(e->graphExec, e->stream));
   return NSF_OK;
 }
@@ -458,9 +459,11 @@ nsf_status nsf_ensemble_march_timed(nsf_ensemble* e, uint64_t nsteps, double* ms
   CKE(cudaEventCreate(&a));
   CKE(cudaEventCreate(&b));
   CKE(cudaEventRecord(a, e->stream));
+  nsf_steps_queued(e->members[0]);
   for (uint64_t q = 0; q < nsteps; ++q) CKE(cudaGraphLaunch(e->graphExec, e->stream));
   CKE(cudaEventRecord(b, e->stream));
   CKE(cudaEventSynchronize(b));
+  nsf_steps_waited(e->members[0]);
   float f = 0;
   CKE(cudaEventElapsedTime(&f, a, b));
   *ms = f;
@@ -501,6 +504,7 @@ nsf_status nsf_ensemble_sync(nsf_ensemble* e) {
   if (!e) return NSF_ERR_ARG;
   if (!e->graphExec) return NSF_ERR_STATE;
   CKE(cudaStreamSynchronize(e->stream));
+  nsf_steps_waited(e->members[0]);
   for (size_t m = 0; m < e->members.size(); ++m) {
     nsf_status st = nsf_sync(e->members[m]);
     if (st != NSF_OK) {
@@ -514,6 +518,7 @@ nsf_status nsf_ensemble_sync(nsf_ensemble* e) {
 nsf_status nsf_ensemble_member(nsf_ensemble* e, uint32_t m, nsf_solver** member) {
   if (!e || !member || m >= e->members.size() || !e->graphExec) return NSF_ERR_ARG;
   CKE(cudaStreamSynchronize(e->stream));  // the member's own calls then see the ensemble's steps
+  nsf_steps_waited(e->members[0]);
   *member = e->members[m];
   return NSF_OK;
 }

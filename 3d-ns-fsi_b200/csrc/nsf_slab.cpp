@@ -511,6 +511,7 @@ nsf_status nsf_slab_group_march(nsf_slab_group* g, uint64_t nsteps) {
   if (!g) return NSF_ERR_ARG;
   if (!g->graphExec) return NSF_ERR_STATE;
   CKG(cudaSetDevice(g->device));
+  if (nsteps) nsf_steps_queued(g->slabs[0]);
   for (uint64_t q = 0; q < nsteps; ++q) CKG(cudaGraphLaunch(g->graphExec, g->stream));
   return NSF_OK;
 }
@@ -523,9 +524,11 @@ nsf_status nsf_slab_group_march_timed(nsf_slab_group* g, uint64_t nsteps, double
   CKG(cudaEventCreate(&a));
   CKG(cudaEventCreate(&b));
   CKG(cudaEventRecord(a, g->stream));
+  nsf_steps_queued(g->slabs[0]);
   for (uint64_t q = 0; q < nsteps; ++q) CKG(cudaGraphLaunch(g->graphExec, g->stream));
   CKG(cudaEventRecord(b, g->stream));
   CKG(cudaEventSynchronize(b));
+  nsf_steps_waited(g->slabs[0]);
   float ms = 0;
   CKG(cudaEventElapsedTime(&ms, a, b));
   cudaEventDestroy(a);
@@ -539,6 +542,7 @@ nsf_status nsf_slab_group_sync(nsf_slab_group* g) {
   if (!g->graphExec) return NSF_ERR_STATE;
   CKG(cudaSetDevice(g->device));
   CKG(cudaStreamSynchronize(g->stream));
+  nsf_steps_waited(g->slabs[0]);
   nsf_status worst = NSF_OK;
   for (nsf_solver* s : g->slabs) {
     const nsf_status st = nsf_sync(s);
@@ -555,6 +559,7 @@ nsf_status nsf_slab_group_solver(nsf_slab_group* g, int32_t slab, nsf_solver** s
   if (!g || !s || slab < 0 || slab >= int32_t(g->slabs.size())) return NSF_ERR_ARG;
   CKG(cudaSetDevice(g->device));
   CKG(cudaStreamSynchronize(g->stream));
+  nsf_steps_waited(g->slabs[0]);
   *s = g->slabs[size_t(slab)];
   return NSF_OK;
 }
@@ -572,6 +577,7 @@ nsf_status nsf_slab_group_download(nsf_slab_group* g, uint32_t mask, double* hos
   if (!g || !host || g->slabs.empty()) return NSF_ERR_ARG;
   CKG(cudaSetDevice(g->device));
   CKG(cudaStreamSynchronize(g->stream));
+  nsf_steps_waited(g->slabs[0]);
   // every slab's owned planes straight to their place in the caller's array
   const HostSetup& W = g->whole;
   for (size_t l = 0; l < g->slabs.size(); ++l) {

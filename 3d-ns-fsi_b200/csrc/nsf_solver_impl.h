@@ -56,7 +56,7 @@ struct nsf_solver {
   struct AdjCtx* adj = nullptr;  // discrete-adjoint state (nsf_adjoint.cpp), created on first use
   // member of an ensemble or x-slab group: its steps are queued on the group's stream, not on `stream`
   bool grouped = false;
-  bool marching = false;  // steps of a small grid queued that nobody has waited for yet (counted per device, nsf_capi.cpp)
+  bool marching = false;  // steps queued that nobody has waited for yet (counted per device, nsf_capi.cpp)
   // asynchronous downloads (nsf_download_async): a copy stream and two device staging buffers used in turn,
   // each with the events that mark its snapshot taken (on `stream`) and its copy to the host done (on
   // dlStream); ticket t uses buffer t & 1
@@ -76,6 +76,10 @@ nsf_status nsf_build_device(nsf_solver* s);
 // Queues nsteps steps on the handle's stream (nsf_capi.cpp): the whole-step kernel where the grid has one (with it, the
 // steps may leave their sets on a tape), else one graph launch per step.
 nsf_status nsf_queue_steps(nsf_solver* s, uint64_t nsteps, const nsf::StepTape& tape = {});
+// For groups that queue their members' steps themselves: one member stands for the group among the handles with steps
+// in flight (nsf_capi.cpp).
+void nsf_steps_queued(nsf_solver* s);
+void nsf_steps_waited(nsf_solver* s);
 // The fields of `mask` at the handle's planes first .. first + count - 1 (reference layout) to host + q * pitch for
 // the q-th field (pitch in doubles); waits for the copies (nsf_capi.cpp).
 nsf_status nsf_download_planes(nsf_solver* s, uint32_t mask, size_t first, size_t count, double* host, size_t pitch);

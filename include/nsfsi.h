@@ -113,7 +113,8 @@ nsf_status nsf_initialize(nsf_solver* s);
 
 /* Replaces `nsteps` calls of Solver::marchTimeStep(t, timeLevel) (Solver.cpp:130-167). Asynchronous:
  * the steps are queued on the handle's stream (one CUDA graph per step; for small grids launches of
- * up to 32 steps each, which share the GPU's SMs with other small handles whose steps are in flight). In end_time mode, steps after
+ * up to 32 steps each, which share the GPU's SMs with other small handles whose steps are in flight; beside
+ * steps of large grids, ensembles or slab groups the graphs). In end_time mode, steps after
  * t reaches t_end are no-ops, as Simulation::run (Simulation.cpp:19-30) would not call them. */
 nsf_status nsf_march(nsf_solver* s, uint64_t nsteps);
 
@@ -187,8 +188,9 @@ nsf_status nsf_get_history(nsf_solver* s, uint64_t first, uint64_t count, double
  * grid does not use (nsf_launches_per_step is 1 there). Both advance the solution. */
 nsf_status nsf_march_timed(nsf_solver* s, uint64_t nsteps, double* elapsed_ms);
 nsf_status nsf_profile_steps(nsf_solver* s, uint64_t nsteps, double* stage_ms, double* step_ms);
-/* Kernel launches issued per RK4 step (for instrumentation); 1 for small grids, whose steps share launches (while
- * other small handles' steps are in flight, those above 120,000 nodes use the launch sequence of large grids). */
+/* Kernel launches issued per RK4 step (for instrumentation); 1 for small grids, whose steps share launches (the
+ * launch sequence of large grids is used beside steps of large grids, ensembles or slab groups, and above 120,000 nodes
+ * also beside those of other small handles). */
 nsf_status nsf_launches_per_step(nsf_solver* s, uint64_t* launches);
 
 /* End-of-step metrics for conserved fields the caller keeps in device memory, allocating nothing.

@@ -79,3 +79,53 @@ def test_handles_in_threads_and_an_adjoint_run_beside_them():
     for q in range(3):
         assert np.array_equal(got[q], ref, equal_nan=True)
     assert got["J"] == J and np.array_equal(got["g"][0], gi) and np.array_equal(got["g"][1], gu)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["handle", "ensemble", "slabs"])
+def test_small_handles_beside_large_steps(kind):
+    """Small handles whose steps are queued beside those of a large grid, an ensemble or a slab group, and alone before
+    and after."""
+    small = [config("sphere", (34, 30, 33), 100), config("shipped", (61, 33, 3), 100)]
+    big = config("tgv", (84, 82, 85), 100)
+    ref, big_ref = [], None
+    for c in small:
+        with nsfsi.Solver(c) as s:
+            s.march(24)
+            s.sync()
+            ref.append((s.download(), s.time()))
+    with nsfsi.Solver(big) as s:
+        assert s.launches_per_step() > 1
+        s.march(12)
+        s.sync()
+        big_ref = s.download()
+    large = {"handle": lambda: nsfsi.Solver(big), "ensemble": lambda: nsfsi.Ensemble([big]),
+             "slabs": lambda: nsfsi.SlabGroup(big, 2)}[kind]()
+    hs = [nsfsi.Solver(c) for c in small]
+    try:
+        for s in hs:
+            s.march(4)
+            s.sync()
+        for _ in range(3):
+            for s in hs:
+                s.march(3)
+            large.march(4)
+            for s in hs:
+                s.march(3)
+        large.sync()
+        for s in hs:
+            s.sync()
+        for s in hs:  # expects the large steps again, then finds none
+            s.march(1)
+            s.sync()
+            s.march(1)
+            s.sync()
+        got = large.member(0).download() if kind == "ensemble" else large.download()
+        assert np.array_equal(got, big_ref)
+        for s, (fields, now) in zip(hs, ref):
+            assert s.time() == now
+            assert np.array_equal(s.download(), fields, equal_nan=True)
+    finally:
+        for s in hs:
+            s.close()
+        large.close()
